@@ -1037,8 +1037,9 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
         B2S_DISPATCH_RHS(K, {
             auto spmv_k = [&](const T* in, T* out) {
                 if constexpr (K >= 4 && K % Vec16<T>::width == 0) {
-                    launch_csr_lanes<T, K>(n, rp, ci, v, in, K, out, K, nullptr, nullptr, cs,
-                                           &ctl->all_stopped);
+                    launch_rhs_lanes<T, K, 0>(n, rp, 0, 0, nullptr, nullptr, ci, v, in, K, out,
+                                              K, nullptr, nullptr, max_row_nnz, cs,
+                                              &ctl->all_stopped);
                 } else {
                     with_async_kernel<T, K, (K >= 2)>(lpr, [&](auto kernel) {
                         const int64_t grid = std::min<int64_t>(async_need,

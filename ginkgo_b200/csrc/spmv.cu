@@ -596,48 +596,6 @@ bool lanes_ok(const T* b, int64_t ldb, const T* c, int64_t ldc, int64_t col0,
            vec_ok(static_cast<const T*>(c), ldc, col0, kk);
 }
 
-// Longest Sellp slice (entries per row) for which rows are paired per lane
-// slot with four or more right-hand sides.
-constexpr int64_t kPairMaxSlice = 64;
-
-template <typename T, int K, int FMT>
-void launch_lanes(int64_t n, const int32_t* rp, int64_t w_or_s, int64_t stride,
-                  const uint64_t* sets, const uint64_t* lens, const int32_t* ci,
-                  const T* v, const T* b, int64_t ldb, T* c, int64_t ldc,
-                  const T* alpha, const T* beta, cudaStream_t st,
-                  int64_t max_slice_len = 0)
-{
-    if constexpr (K >= 4 && K % Vec16<T>::width == 0) {
-        constexpr int KL = K / Vec16<T>::width;
-        // Ell: row pairs per lane slot when the column-major layout keeps
-        // rows r, r + 1 adjacent at 8-byte alignment (0.84-0.90 of the
-        // single-row time at 4 and 16 columns on the 7-point 128^3 matrix).
-        // Sellp pairs its rows only when the caller gives the longest slice
-        // and it is short: on the power-law matrix its longest slices (1,805
-        // entries) doubled the per-thread chain and took 1.3 to 2.4 times as
-        // long with pairs.
-        const bool aligned = reinterpret_cast<uintptr_t>(ci) % 8 == 0 &&
-                             reinterpret_cast<uintptr_t>(v) % (2 * sizeof(T)) == 0;
-        // (Sellp FP32 with four columns measured 9 % slower with pairs, so
-        // FP32 pairs need eight or more)
-        const bool pairs = aligned && ((FMT == 1 && stride % 2 == 0) ||
-                                       (FMT == 2 && w_or_s % 2 == 0 && max_slice_len > 0 &&
-                                        max_slice_len <= kPairMaxSlice &&
-                                        (sizeof(T) == 8 || K >= 8)));
-        if (FMT != 0 && pairs) {
-            if constexpr (FMT != 0) {
-                rhs_lanes2_kernel<T, K, FMT><<<ceildiv(ceildiv(n, 2) * KL, kBlock), kBlock, 0,
-                                               st>>>(n, w_or_s, stride, sets, lens, ci, v, b,
-                                                     ldb, c, ldc, alpha, beta);
-            }
-            return;
-        }
-        rhs_lanes_kernel<T, K, FMT><<<ceildiv(n * KL, kBlock), kBlock, 0, st>>>(
-            n, rp, w_or_s, stride, sets, lens, ci, v, b, ldb, c, ldc, alpha,
-            beta);
-    }
-}
-
 #define B2S_DISPATCH_K(kk, VEC, ...)                   \
     switch (kk) {                                      \
     case 16: { constexpr int K = 16; __VA_ARGS__; break; } \
@@ -749,8 +707,10 @@ int csr_spmv(int strategy, int64_t n, int64_t num_cols, const int32_t* rp,
             });
         } else if (lanes_ok(b, ldb, c, ldc, col0, kk)) {
             B2S_DISPATCH_K(kk, VEC, {
-                launch_lanes<T, K, 0>(n, rp, 0, 0, nullptr, nullptr, ci, v, bb,
-                                      ldb, cc, ldc, alpha, beta, st);
+                if constexpr (K >= 4 && K % Vec16<T>::width == 0) {
+                    launch_rhs_lanes<T, K, 0>(n, rp, 0, 0, nullptr, nullptr, ci, v, bb, ldb,
+                                              cc, ldc, alpha, beta, max_row_nnz, st);
+                }
             });
         } else if (kk <= 2) {
             // persistent: as many blocks as fit on the SMs at once; rows of
@@ -820,9 +780,11 @@ int ell_spmv(int64_t n, int64_t num_cols, int64_t width, int64_t stride,
         const bool vec = vec_ok(b, ldb, col0, kk);
         if (lanes_ok(b, ldb, c, ldc, col0, kk)) {
             B2S_DISPATCH_K(kk, VEC, {
-                launch_lanes<T, K, 1>(n, nullptr, width, stride, nullptr,
-                                      nullptr, ci, v, b + col0, ldb, c + col0,
-                                      ldc, alpha, beta, st);
+                if constexpr (K >= 4 && K % Vec16<T>::width == 0) {
+                    launch_rhs_lanes<T, K, 1>(n, nullptr, width, stride, nullptr, nullptr, ci, v,
+                                              b + col0, ldb, c + col0, ldc, alpha, beta, width,
+                                              st);
+                }
             });
             B2S_LAUNCH_CHECK();
             col0 += kk;
@@ -899,9 +861,11 @@ int sellp_spmv(int64_t n, int64_t num_cols, int64_t slice_size,
         const bool vec = vec_ok(b, ldb, col0, kk);
         if (lanes_ok(b, ldb, c, ldc, col0, kk)) {
             B2S_DISPATCH_K(kk, VEC, {
-                launch_lanes<T, K, 2>(n, nullptr, slice_size, 0, slice_sets,
-                                      slice_lengths, ci, v, b + col0, ldb,
-                                      c + col0, ldc, alpha, beta, st, max_slice_len);
+                if constexpr (K >= 4 && K % Vec16<T>::width == 0) {
+                    launch_rhs_lanes<T, K, 2>(n, nullptr, slice_size, 0, slice_sets,
+                                              slice_lengths, ci, v, b + col0, ldb, c + col0, ldc,
+                                              alpha, beta, max_slice_len, st);
+                }
             });
             B2S_LAUNCH_CHECK();
             col0 += kk;

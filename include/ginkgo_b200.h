@@ -119,7 +119,7 @@ int b2s_sellp_spmv_f32(int64_t num_rows, int64_t num_cols, int64_t slice_size,
 /* The same with the caller's knowledge of the longest slice
  * (max_slice_length = the largest slice_lengths entry; 0 when not known):
  * with four or more right-hand sides, slices of at most 64 entries per row
- * let each lane slot take two neighbouring rows. */
+ * let a warp take several rows together. */
 int b2s_sellp_spmv_hinted_f64(int64_t num_rows, int64_t num_cols, int64_t slice_size,
                               const uint64_t* slice_sets, const uint64_t* slice_lengths,
                               const int32_t* col_idxs, const double* values, const double* b,
