@@ -94,14 +94,23 @@ struct __align__(16) AsyncStage {
     int32_t cols[kAsyncCap];
 };
 
-template <typename T, int K, bool VEC, int LPR = 1>
-__global__ void __launch_bounds__(kAsyncBlock)
-    csr_async_kernel(int64_t n, const int32_t* __restrict__ rp,
-                     const int32_t* __restrict__ ci, const T* __restrict__ v,
-                     const T* __restrict__ b, int64_t ldb, T* __restrict__ c,
-                     int64_t ldc, const T* __restrict__ alpha,
-                     const T* __restrict__ beta,
-                     const int* __restrict__ skip = nullptr)
+// What a solver does with the finished rows: row() sees each row's sums in
+// the lane that stores them, finish() runs once per thread after the last
+// row, all threads of the block together, with the block's shared memory.
+struct NoEpilogue {
+    static constexpr bool kOn = false;
+    template <typename T>
+    __device__ __forceinline__ void row(int64_t, T)
+    {}
+    __device__ __forceinline__ void finish(void*) {}
+};
+
+template <typename T, int K, bool VEC, int LPR, typename Epi>
+__device__ __forceinline__ void csr_async_rows(
+    int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+    const T* __restrict__ v, const T* __restrict__ b, int64_t ldb, T* __restrict__ c,
+    int64_t ldc, const T* __restrict__ alpha, const T* __restrict__ beta,
+    const int* __restrict__ skip, Epi epi)
 {
     static_assert(LPR >= 1 && LPR <= 32 && (32 % LPR) == 0, "LPR divides 32");
     constexpr unsigned kFull = 0xffffffffu;
@@ -137,11 +146,13 @@ __global__ void __launch_bounds__(kAsyncBlock)
     };
     if (skip != nullptr && *skip) return;  // whole grid (solver idle)
     int64_t g = blockIdx.x * int64_t(kAsyncBlock / kWarp) + wid;
-    if (g >= ngroups) return;  // whole warp
-    int rs, re, start, cnt, p, pe;
-    load_ptrs(g, p, pe);
-    desc(p, pe, rs, re, start, cnt);
-    if (cnt <= kCap) issue(0, start, cnt);
+    if (!Epi::kOn && g >= ngroups) return;  // whole warp
+    int rs = 0, re = 0, start = 0, cnt = 0, p, pe;
+    if (!Epi::kOn || g < ngroups) {
+        load_ptrs(g, p, pe);
+        desc(p, pe, rs, re, start, cnt);
+        if (cnt <= kCap) issue(0, start, cnt);
+    }
     cp_async_commit();
     // pointers of the group after the next
     int pn = 0, pen = 0;
@@ -204,6 +215,9 @@ __global__ void __launch_bounds__(kAsyncBlock)
             for (int j = 0; j < K; ++j) {
                 if (j % LPR == sub) dst[j] = combine(acc[j], alpha, beta, dst + j);
             }
+            if constexpr (Epi::kOn && K == 1) {
+                if (sub == 0) epi.row(row, acc[0]);
+            }
         }
         __syncwarp();  // stage s is refilled two groups later
         s ^= 1;
@@ -212,6 +226,34 @@ __global__ void __launch_bounds__(kAsyncBlock)
         start = nstart;
         cnt = ncnt;
     }
+    if constexpr (Epi::kOn) {
+        __syncthreads();
+        epi.finish(stages);
+    }
+}
+
+template <typename T, int K, bool VEC, int LPR = 1>
+__global__ void __launch_bounds__(kAsyncBlock)
+    csr_async_kernel(int64_t n, const int32_t* __restrict__ rp,
+                     const int32_t* __restrict__ ci, const T* __restrict__ v,
+                     const T* __restrict__ b, int64_t ldb, T* __restrict__ c,
+                     int64_t ldc, const T* __restrict__ alpha,
+                     const T* __restrict__ beta,
+                     const int* __restrict__ skip = nullptr)
+{
+    csr_async_rows<T, K, VEC, LPR>(n, rp, ci, v, b, ldb, c, ldc, alpha, beta, skip,
+                                   NoEpilogue());
+}
+
+// c = A b for one column, with a solver's epilogue.
+template <typename T, int LPR, typename Epi>
+__global__ void __launch_bounds__(kAsyncBlock, 4)
+    csr_async_epi_kernel(int64_t n, const int32_t* __restrict__ rp,
+                         const int32_t* __restrict__ ci, const T* __restrict__ v,
+                         const T* __restrict__ b, T* __restrict__ c,
+                         const int* __restrict__ skip, Epi epi)
+{
+    csr_async_rows<T, 1, false, LPR>(n, rp, ci, v, b, 1, c, 1, nullptr, nullptr, skip, epi);
 }
 
 // Calls f(csr_async_kernel<T, K, VEC, LPR>) for the runtime lanes-per-row
@@ -225,6 +267,14 @@ void with_async_kernel(int lpr, F&& f)
     default: f(csr_async_kernel<T, K, VEC, 4>); break;
     }
 }
-
+template <typename T, typename Epi, typename F>
+void with_async_epi_kernel(int lpr, F&& f)
+{
+    switch (lpr) {
+    case 1: f(csr_async_epi_kernel<T, 1, Epi>); break;
+    case 2: f(csr_async_epi_kernel<T, 2, Epi>); break;
+    default: f(csr_async_epi_kernel<T, 4, Epi>); break;
+    }
+}
 
 }  // namespace b2s

@@ -69,6 +69,7 @@ struct SolveCtl {
     double reduction;  // residual goal relative to the baseline
     int baseline;      // B2S_BASELINE_*: ||b||, ||r_0|| or 1
     int implicit;      // stop::ImplicitResidualNorm: sqrt|rho| instead of ||r||
+    int failed;        // a kernel gave up waiting for its other blocks
     uint8_t status[kMaxRhs];
 };
 
