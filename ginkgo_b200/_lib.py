@@ -90,9 +90,16 @@ def lib():
     return _lib
 
 
+_entries = {}
+
+
 def call(name, *args):
-    """Calls an int-returning entry point and raises on a negative status."""
-    rc = getattr(lib(), name)(*args)
+    """Calls an int-returning entry point and raises on a negative status.
+    Pointer arguments may be plain integers (tensor.data_ptr())."""
+    f = _entries.get(name)
+    if f is None:
+        f = _entries[name] = getattr(lib(), name)
+    rc = f(*args)
     if rc < 0:
         msg = lib().b2s_last_error().decode(errors="replace")
         raise GinkgoError(name, rc, msg)

@@ -42,11 +42,12 @@ class CudaExecutor:
 
 
 def _stream(t: torch.Tensor):
-    return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    # the handle alone: a torch.cuda.Stream object costs about 1.5 us
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
 def _p(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _as2d(t: torch.Tensor):
@@ -71,10 +72,22 @@ def _check_dense(t: torch.Tensor, rows: int, dtype, what: str):
     return t2
 
 
+def _dense_layout(t: torch.Tensor, rows: int, dtype, what: str):
+    """(leading dimension, columns) of an operand; _check_dense's rules
+    without a 2-D view of a vector."""
+    if t.dim() == 1 and t.is_cuda and t.shape[0] == rows and \
+            (t.dtype == dtype or (dtype is None and t.dtype in _SFX)):
+        return t.stride(0), 1
+    t2 = _check_dense(t, rows, dtype, what)
+    return t2.stride(0), t2.shape[1]
+
+
 def _scalar(v, dtype, device):
     if v is None:
         return None
     if isinstance(v, torch.Tensor):
+        if v.dtype == dtype and v.device == device and v.numel() == 1:
+            return v
         return v.to(device=device, dtype=dtype).reshape(1)
     return torch.tensor([v], dtype=dtype, device=device)
 
@@ -84,9 +97,9 @@ class _SparseBase:
     shape: tuple
 
     def _apply_args(self, args, mixed=False):
-        """(b, x, alpha, beta) as 2-D views; with mixed, b and x may each be
-        FP64 or FP32 (alpha then has the matrix type, beta the type of x, as
-        core/matrix/csr.cpp:301-311 converts them)."""
+        """(b, x, alpha, beta, ldb, ldx, columns); with mixed, b and x may
+        each be FP64 or FP32 (alpha then has the matrix type, beta the type of
+        x, as core/matrix/csr.cpp:301-311 converts them)."""
         if len(args) == 2:
             b, x = args
             alpha = beta = None
@@ -95,16 +108,17 @@ class _SparseBase:
         else:
             raise TypeError("apply(b, x) or apply(alpha, b, beta, x)")
         n, m = self.shape
-        b2 = _check_dense(b, m, None if mixed else self.dtype, "b")
-        x2 = _check_dense(x, n, None if mixed else self.dtype, "x")
-        if b2.shape[1] != x2.shape[1]:
+        ldb, kb = _dense_layout(b, m, None if mixed else self.dtype, "b")
+        ldx, kx = _dense_layout(x, n, None if mixed else self.dtype, "x")
+        if kb != kx:
             raise ValueError("b and x have different numbers of columns")
-        dev = x2.device
-        return (b2, x2, _scalar(alpha, self.dtype, dev),
-                _scalar(beta, x2.dtype, dev))
+        if alpha is not None or beta is not None:
+            alpha = _scalar(alpha, self.dtype, x.device)
+            beta = _scalar(beta, x.dtype, x.device)
+        return b, x, alpha, beta, ldb, ldx, kx
 
-    def _uniform(self, b2, x2):
-        return b2.dtype == self.dtype and x2.dtype == self.dtype
+    def _uniform(self, b, x):
+        return b.dtype == self.dtype and x.dtype == self.dtype
 
 
 class Csr(_SparseBase):
@@ -174,20 +188,20 @@ class Csr(_SparseBase):
         b = args[1] if len(args) == 4 else args[0]
         if isinstance(b, (Csr, Identity)):
             return self._apply_sparse(args)
-        b2, x2, alpha, beta = self._apply_args(args, mixed=True)
+        b2, x2, alpha, beta, ldb, ldx, k = self._apply_args(args, mixed=True)
         if not self._uniform(b2, x2):
             call("b2s_csr_spmv_mixed", _VT[self.dtype], _VT[b2.dtype], _VT[x2.dtype],
                  self.shape[0], self.shape[1], _p(self.row_ptrs), _p(self.col_idxs),
-                 _p(self.values), self.max_row_nnz, _p(b2), b2.stride(0), _p(x2),
-                 x2.stride(0), x2.shape[1], _p(alpha), _p(beta), _stream(x2))
+                 _p(self.values), self.max_row_nnz, _p(b2), ldb, _p(x2), ldx, k, _p(alpha),
+                 _p(beta), _stream(x2))
             return args[-1]
         strat = 1 if self.strategy == "load_balance" else 0
         nt = 0 if self._tiles is None else self._tiles.numel() - 1
         call(f"b2s_csr_spmv_{_SFX[self.dtype]}", strat, self.shape[0],
              self.shape[1], _p(self.row_ptrs), _p(self.col_idxs),
              _p(self.values), self.max_row_nnz if strat == 0 else 0,
-             _p(self._tiles), nt, _p(b2), b2.stride(0), _p(x2), x2.stride(0),
-             x2.shape[1], _p(alpha), _p(beta), _stream(x2))
+             _p(self._tiles), nt, _p(b2), ldb, _p(x2), ldx, k, _p(alpha), _p(beta),
+             _stream(x2))
         return args[-1]
 
     def _apply_sparse(self, args):
@@ -300,17 +314,16 @@ class Ell(_SparseBase):
 
     def apply(self, *args):
         """As Csr.apply: b and x may each be FP64 or FP32."""
-        b2, x2, alpha, beta = self._apply_args(args, mixed=True)
+        b2, x2, alpha, beta, ldb, ldx, k = self._apply_args(args, mixed=True)
         if not self._uniform(b2, x2):
             call("b2s_ell_spmv_mixed", _VT[self.dtype], _VT[b2.dtype], _VT[x2.dtype],
                  self.shape[0], self.shape[1], self.width, self.stride,
-                 _p(self.col_idxs), _p(self.values), _p(b2), b2.stride(0), _p(x2),
-                 x2.stride(0), x2.shape[1], _p(alpha), _p(beta), _stream(x2))
+                 _p(self.col_idxs), _p(self.values), _p(b2), ldb, _p(x2), ldx, k, _p(alpha),
+                 _p(beta), _stream(x2))
             return args[-1]
         call(f"b2s_ell_spmv_{_SFX[self.dtype]}", self.shape[0], self.shape[1],
-             self.width, self.stride, _p(self.col_idxs), _p(self.values),
-             _p(b2), b2.stride(0), _p(x2), x2.stride(0), x2.shape[1],
-             _p(alpha), _p(beta), _stream(x2))
+             self.width, self.stride, _p(self.col_idxs), _p(self.values), _p(b2), ldb, _p(x2),
+             ldx, k, _p(alpha), _p(beta), _stream(x2))
         return args[-1]
 
 
@@ -337,19 +350,22 @@ class Sellp(_SparseBase):
     def apply(self, *args):
         """Operands of another type are converted to the matrix type and the
         result back (precision_dispatch, core/matrix/sellp.cpp:150-180)."""
-        b2, x2, alpha, beta = self._apply_args(args, mixed=True)
+        b2, x2, alpha, beta, ldb, ldx, k = self._apply_args(args, mixed=True)
         bt, xt = b2, x2
+        if not self._uniform(b2, x2):
+            bt, xt = b2, x2 = _as2d(b2), _as2d(x2)
         if b2.dtype != self.dtype:
             bt = _convert(b2, self.dtype)
+            ldb = bt.stride(0)
         if x2.dtype != self.dtype:
             xt = _convert(x2, self.dtype) if beta is not None else \
                 torch.empty(x2.shape, dtype=self.dtype, device=x2.device)
             beta = None if beta is None else beta.to(self.dtype)
+            ldx = xt.stride(0)
         call(f"b2s_sellp_spmv_hinted_{_SFX[self.dtype]}", self.shape[0], self.shape[1],
              self.slice_size, _p(self.slice_sets), _p(self.slice_lengths),
-             _p(self.col_idxs), _p(self.values), _p(bt), bt.stride(0), _p(xt),
-             xt.stride(0), xt.shape[1], _p(alpha), _p(beta), self.max_slice_length,
-             _stream(xt))
+             _p(self.col_idxs), _p(self.values), _p(bt), ldb, _p(xt), ldx, k, _p(alpha),
+             _p(beta), self.max_slice_length, _stream(xt))
         if xt is not x2:
             call("b2s_dense_convert", _VT[xt.dtype], _VT[x2.dtype], x2.shape[0], x2.shape[1],
                  _p(xt), xt.stride(0), _p(x2), x2.stride(0), _stream(x2))
@@ -450,12 +466,12 @@ class Hybrid(_SparseBase):
         return int(self.coo_values.numel())
 
     def apply(self, *args):
-        b2, x2, alpha, beta = self._apply_args(args)
+        b2, x2, alpha, beta, ldb, ldx, k = self._apply_args(args)
         call(f"b2s_hybrid_spmv_{_SFX[self.dtype]}", self.shape[0], self.shape[1],
              self.width, self.stride, _p(self.ell_col_idxs), _p(self.ell_values),
              self.coo_nnz, _p(self.coo_row_idxs), _p(self.coo_col_idxs),
-             _p(self.coo_values), _p(b2), b2.stride(0), _p(x2), x2.stride(0), x2.shape[1],
-             _p(alpha), _p(beta), _stream(x2))
+             _p(self.coo_values), _p(b2), ldb, _p(x2), ldx, k, _p(alpha), _p(beta),
+             _stream(x2))
         return args[-1]
 
     def convert_to_csr(self) -> Csr:
