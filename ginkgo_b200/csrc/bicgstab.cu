@@ -58,35 +58,47 @@ __device__ __forceinline__ T bicg_s(T r, T v, T alpha)
     return add_rn(r, -mul_rn(alpha, v));
 }
 
-// The last block's part of the update pass (thread 0): tot holds dot(rr, r)
+// The last block's part of the update pass (its first warp, lane j taking
+// column j, every load issued before the first store): tot holds dot(rr, r)
 // and ||r||^2 per column; finalises the columns that stopped at s, advances
 // the iteration, swaps rho and applies the checks.
 template <typename T, int K>
 __device__ void bicg_update_finish(const T* tot, SolveCtl* ctl, BicgScalars<T>* sc)
 {
-    ctl->ticket = 0;
-    int all_after_s = 1;
-    for (int j = 0; j < K; ++j) all_after_s &= has_stopped(ctl->status[j]);
-    const int iter = all_after_s ? ctl->iter : ctl->iter + 1;
-    ctl->iter = iter;
-    int all = 1;
-    for (int j = 0; j < K; ++j) {
-        uint8_t st = ctl->status[j];
-        if (has_stopped(st)) {
+    const int j = threadIdx.x;
+    const int iter0 = ctl->iter, max_iters = ctl->max_iters;
+    uint8_t st = 0;
+    T old_rho = T(0), rho = T(0), tau = T(0);
+    bool met = false, was = true;
+    if (j < K) {
+        st = ctl->status[j];
+        old_rho = sc->rho[j];
+        rho = tot[j];
+        tau = sqrt(tot[K + j]);
+        met = residual_met(ctl, tau, rho, sc->start[j]);
+        was = has_stopped(st);
+    }
+    const int iter = __all_sync(0xffffffffu, was) ? iter0 : iter0 + 1;
+    bool stopped = true;
+    if (j < K) {
+        if (was) {
             st |= kFinalizedMask;
         } else {
-            sc->prev_rho[j] = sc->rho[j];
-            sc->rho[j] = tot[j];
-            sc->tau[j] = sqrt(tot[K + j]);
-            if (residual_met(ctl, sc->tau[j], sc->rho[j], sc->start[j])) {
-                converge_status(st, kResidualId, true);
-            }
-            if (iter >= ctl->max_iters) stop_status(st, kIterationId, true);
+            if (met) converge_status(st, kResidualId, true);
+            if (iter >= max_iters) stop_status(st, kIterationId, true);
+            sc->prev_rho[j] = old_rho;
+            sc->rho[j] = rho;
+            sc->tau[j] = tau;
         }
         ctl->status[j] = st;
-        all &= has_stopped(st);
+        stopped = has_stopped(st);
     }
-    ctl->all_stopped = all;
+    const bool all = __all_sync(0xffffffffu, stopped);
+    if (j == 0) {
+        ctl->ticket = 0;
+        ctl->iter = iter;
+        ctl->all_stopped = all;
+    }
 }
 
 // The last block's part of the pass after the first SpMV (thread j < K):
@@ -102,25 +114,27 @@ __device__ void bicg_alpha_finish(const T* tot, SolveCtl* ctl, BicgScalars<T>* s
     if (threadIdx.x == 0) ctl->ticket = 0;
 }
 
-// The last block's part of the pass after the second SpMV (thread 0): tot
-// holds dot(s, t), dot(t, t) and ||s||^2 per column; the check on s
+// The last block's part of the pass after the second SpMV (thread j < K):
+// tot holds dot(s, t), dot(t, t) and ||s||^2 per column; the check on s
 // (without finalising: the update pass adds alpha y) and omega.
 template <typename T, int K>
 __device__ void bicg_omega_finish(const T* tot, SolveCtl* ctl, BicgScalars<T>* sc)
 {
-    ctl->ticket = 0;
-    for (int j = 0; j < K; ++j) {
+    const int j = threadIdx.x;
+    if (j < K) {
         uint8_t st = ctl->status[j];
-        if (has_stopped(st)) continue;
-        const T tau_s = sqrt(tot[2 * K + j]);
-        if (residual_met(ctl, tau_s, sc->rho[j], sc->start[j])) {
-            converge_status(st, kResidualId, false);
-            sc->tau[j] = tau_s;
+        const T tau_s = sqrt(tot[2 * K + j]), tt = tot[K + j];
+        const bool met = residual_met(ctl, tau_s, sc->rho[j], sc->start[j]);
+        if (!has_stopped(st)) {
+            if (met) {
+                converge_status(st, kResidualId, false);
+                sc->tau[j] = tau_s;
+            }
+            ctl->status[j] = st;
+            sc->omega[j] = tt != T(0) ? tot[j] / tt : T(0);
         }
-        ctl->status[j] = st;
-        const T tt = tot[K + j];
-        sc->omega[j] = tt != T(0) ? tot[j] / tt : T(0);
     }
+    if (j == 0) ctl->ticket = 0;
 }
 
 template <typename T, int K>
@@ -322,23 +336,7 @@ __global__ void __launch_bounds__(kSolverBlock)
     block_partials<T, 3 * K>(acc3, partials, red);
     if (last_block_done(&ctl->ticket, &last)) {
         sum_partials<T, 3 * K>(partials, gridDim.x, tot, red);
-        if (threadIdx.x == 0) {
-            ctl->ticket = 0;
-            for (int j = 0; j < K; ++j) {
-                uint8_t st = ctl->status[j];
-                if (has_stopped(st)) continue;
-                const T tau_s = sqrt(tot[2 * K + j]);
-                // check on s without finalising (core/solver/bicgstab.cpp
-                // second check): the update pass adds alpha y and finalises
-                if (residual_met(ctl, tau_s, sc->rho[j], sc->start[j])) {
-                    converge_status(st, kResidualId, false);
-                    sc->tau[j] = tau_s;
-                }
-                ctl->status[j] = st;
-                const T tt = tot[K + j];
-                sc->omega[j] = tt != T(0) ? tot[j] / tt : T(0);
-            }
-        }
+        bicg_omega_finish<T, K>(tot, ctl, sc);
     }
 }
 
@@ -390,7 +388,7 @@ __global__ void __launch_bounds__(kSolverBlock)
     block_partials<T, 2 * K>(acc, partials, red);
     if (last_block_done(&ctl->ticket, &last)) {
         sum_partials<T, 2 * K>(partials, gridDim.x, tot, red);
-        if (threadIdx.x == 0) bicg_update_finish<T, K>(tot, ctl, sc);
+        if (threadIdx.x < kWarp) bicg_update_finish<T, K>(tot, ctl, sc);
     }
 }
 
@@ -415,30 +413,44 @@ __global__ void __launch_bounds__(kSolverBlock)
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kSolverBlock)
-    bicg_dot1_kernel(int64_t n, const T* __restrict__ rr, const T* __restrict__ v,
-                     SolveCtl* ctl, BicgScalars<T>* sc, T* __restrict__ partials)
-{
-    __shared__ T red[kSolverBlock / kWarp];
-    __shared__ T tot[1];
-    __shared__ int last;
-    if (ctl->all_stopped) return;
-    T acc[1] = {T(0)};
-    for (int64_t i = blockIdx.x * int64_t(kSolverBlock) + threadIdx.x; i < n;
-         i += int64_t(gridDim.x) * kSolverBlock) {
-        acc[0] += rr[i] * v[i];
-    }
-    block_partials<T, 1>(acc, partials, red);
-    if (last_block_done(&ctl->ticket, &last)) {
-        sum_partials<T, 1>(partials, gridDim.x, tot, red);
-        if (threadIdx.x == 0) {
-            const T bv = tot[0];
-            sc->alpha[0] = bv != T(0) ? sc->rho[0] / bv : T(0);
-            ctl->ticket = 0;
+// Epilogue of csr_async_epi_kernel: the dots that follow each SpMV, from the
+// rows as they finish.  NS = 1: a = r_hat, dot(a, q) -> alpha; NS = 3: a = s,
+// dot(a, q), dot(q, q), ||a||^2 -> the check on s and omega.
+template <typename T, int NS>
+struct BicgDotEpilogue {
+    static constexpr bool kOn = true;
+    const T* a;
+    T* partials;
+    SolveCtl* ctl;
+    BicgScalars<T>* sc;
+    T sum[NS] = {};
+    __device__ __forceinline__ void row(int64_t i, T q)
+    {
+        const T ai = a[i];
+        sum[0] += ai * q;
+        if constexpr (NS == 3) {
+            sum[1] += q * q;
+            sum[2] += ai * ai;
         }
     }
-}
+    // sm: the block's stages, no longer used
+    __device__ __forceinline__ void finish(void* sm)
+    {
+        static_assert(kAsyncBlock == kSolverBlock, "one block size");
+        T* red = static_cast<T*>(sm);
+        T* tot = red + NS * kSolverBlock / kWarp;
+        int* last = reinterpret_cast<int*>(tot + NS);
+        block_partials<T, NS>(sum, partials, red);
+        if (last_block_done(&ctl->ticket, last)) {
+            sum_partials<T, NS>(partials, gridDim.x, tot, red);
+            if constexpr (NS == 1) {
+                bicg_alpha_finish<T, 1>(tot, ctl, sc);
+            } else {
+                bicg_omega_finish<T, 1>(tot, ctl, sc);
+            }
+        }
+    }
+};
 
 template <typename T>
 __global__ void __launch_bounds__(kSolverBlock)
@@ -453,43 +465,6 @@ __global__ void __launch_bounds__(kSolverBlock)
         const T sr = bicg_s(r[i], v[i], alpha);
         s[i] = sr;
         z[i] = dinv ? mul_rn(dinv[i], sr) : sr;
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kSolverBlock)
-    bicg_dot2_kernel(int64_t n, const T* __restrict__ s, const T* __restrict__ t,
-                     SolveCtl* ctl, BicgScalars<T>* sc, T* __restrict__ partials)
-{
-    __shared__ T red[kSolverBlock / kWarp * 3];
-    __shared__ T tot[3];
-    __shared__ int last;
-    if (ctl->all_stopped) return;
-    T acc[3] = {T(0), T(0), T(0)};
-    for (int64_t i = blockIdx.x * int64_t(kSolverBlock) + threadIdx.x; i < n;
-         i += int64_t(gridDim.x) * kSolverBlock) {
-        const T si = s[i], ti = t[i];
-        acc[0] += si * ti;
-        acc[1] += ti * ti;
-        acc[2] += si * si;
-    }
-    block_partials<T, 3>(acc, partials, red);
-    if (last_block_done(&ctl->ticket, &last)) {
-        sum_partials<T, 3>(partials, gridDim.x, tot, red);
-        if (threadIdx.x == 0) {
-            ctl->ticket = 0;
-            uint8_t st = ctl->status[0];
-            if (!has_stopped(st)) {
-                const T tau_s = sqrt(tot[2]);
-                // the check on s without finalising, as in bicg_spmv2_kernel
-                if (residual_met(ctl, tau_s, sc->rho[0], sc->start[0])) {
-                    converge_status(st, kResidualId, false);
-                    sc->tau[0] = tau_s;
-                }
-                ctl->status[0] = st;
-                sc->omega[0] = tot[1] != T(0) ? tot[0] / tot[1] : T(0);
-            }
-        }
     }
 }
 
@@ -632,16 +607,6 @@ __device__ __forceinline__ void lanes_partials(T (&acc)[NS][int(16 / sizeof(T))]
     }
 }
 
-// The last block: tot[m * K + j] = sum over blocks of partials[m][.][j].
-template <typename T, int K, int NS>
-__device__ __forceinline__ void lanes_totals(const T* __restrict__ partials, T* tot, T* red)
-{
-#pragma unroll
-    for (int m = 0; m < NS; ++m) {
-        sum_partials<T, K>(partials + int64_t(m) * gridDim.x * K, gridDim.x, tot + m * K, red);
-    }
-}
-
 // NS = 1: dot(rr, v) -> alpha; NS = 3: dot(s, t), dot(t, t), ||s||^2 ->
 // the check on s and omega
 template <typename T, int K, int NS>
@@ -679,11 +644,67 @@ __global__ void __launch_bounds__(kSolverBlock)
     }
     lanes_partials<T, K, NS>(acc, col0, partials, red);
     if (last_block_done(&ctl->ticket, &last)) {
-        lanes_totals<T, K, NS>(partials, tot, red);
+        fold_columns<T, K, NS>(partials, gridDim.x, tot);
         if constexpr (NS == 1) {
             bicg_alpha_finish<T, K>(tot, ctl, sc);
         } else {
-            if (threadIdx.x == 0) bicg_omega_finish<T, K>(tot, ctl, sc);
+            bicg_omega_finish<T, K>(tot, ctl, sc);
+        }
+    }
+}
+
+// q = A in for K columns, a warp per ROWS rows (rhs_rows), with the dots of
+// bicg_dots_lanes_kernel from the finished rows.
+// 20 iterations of the 2D convection-diffusion step, before -> with this pass
+// and the columns' scalars side by side: 128^2 4 columns 1.23 -> 0.98 ms, 16
+// columns 2.19 -> 1.11 ms; 724^2 2.79 -> 2.45 and 8.65 -> 7.22 ms.
+template <typename T, int K, int ROWS, int NS>
+__global__ void __launch_bounds__(kSolverBlock)
+    bicg_spmv_rows_kernel(int64_t n, const int32_t* __restrict__ rp,
+                          const int32_t* __restrict__ ci, const T* __restrict__ v,
+                          const T* __restrict__ in, T* __restrict__ q,
+                          const T* __restrict__ a, SolveCtl* ctl, BicgScalars<T>* sc,
+                          T* __restrict__ partials)
+{
+    constexpr int VW = int(16 / sizeof(T));
+    constexpr int KL = K / VW;
+    constexpr int W = kSolverBlock / kWarp;
+    __shared__ T red[W * NS * K];
+    __shared__ T tot[NS * K];
+    __shared__ int last;
+    if (ctl->all_stopped) return;
+    T acc[NS][VW];
+#pragma unroll
+    for (int m = 0; m < NS; ++m) {
+#pragma unroll
+        for (int u = 0; u < VW; ++u) acc[m][u] = T(0);
+    }
+    const int64_t step = int64_t(gridDim.x) * W * ROWS;
+    for (int64_t r0 = (blockIdx.x * int64_t(W) + threadIdx.x / kWarp) * ROWS; r0 < n; r0 += step) {
+        rhs_rows<T, K, 0, ROWS>(
+            n, r0, rp, 0, 0, nullptr, nullptr, ci, v, in, K,
+            [&](int64_t row, int col0, const typename Vec16<T>::type& sum) {
+                T qv[VW], av[VW];
+                memcpy(qv, &sum, 16);
+                ld_vec<T, VW>(a + row * K + col0, av);
+#pragma unroll
+                for (int u = 0; u < VW; ++u) {
+                    acc[0][u] += av[u] * qv[u];
+                    if constexpr (NS == 3) {
+                        acc[1][u] += qv[u] * qv[u];
+                        acc[2][u] += av[u] * av[u];
+                    }
+                }
+                st_vec<T, VW>(q + row * K + col0, qv);
+            });
+    }
+    lanes_partials<T, K, NS>(acc, int(threadIdx.x % KL) * VW, partials, red);
+    if (last_block_done(&ctl->ticket, &last)) {
+        fold_columns<T, K, NS>(partials, gridDim.x, tot);
+        if constexpr (NS == 1) {
+            bicg_alpha_finish<T, K>(tot, ctl, sc);
+        } else {
+            bicg_omega_finish<T, K>(tot, ctl, sc);
         }
     }
 }
@@ -745,8 +766,8 @@ __global__ void __launch_bounds__(kSolverBlock)
     }
     lanes_partials<T, K, 2>(acc, col0, partials, red);
     if (last_block_done(&ctl->ticket, &last)) {
-        lanes_totals<T, K, 2>(partials, tot, red);
-        if (threadIdx.x == 0) bicg_update_finish<T, K>(tot, ctl, sc);
+        fold_columns<T, K, 2>(partials, gridDim.x, tot);
+        if (threadIdx.x < kWarp) bicg_update_finish<T, K>(tot, ctl, sc);
     }
 }
 
@@ -884,7 +905,7 @@ __global__ void __launch_bounds__(kSolverBlock)
     block_partials<T, 3 * K>(acc, partials, red);
     if (last_block_done(&ctl->ticket, &last)) {
         sum_partials<T, 3 * K>(partials, gridDim.x, tot, red);
-        if (threadIdx.x == 0) bicg_omega_finish<T, K>(tot, ctl, sc);
+        bicg_omega_finish<T, K>(tot, ctl, sc);
     }
 }
 
@@ -1021,13 +1042,17 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
     // the split single-RHS passes (large systems)
     const int lpr = async_lanes_per_row(max_row_nnz);
     const int64_t async_need = ceildiv(ceildiv(n, kWarp / lpr), kAsyncBlock / kWarp);
-    auto async_spmv = [&](cudaStream_t cs, const T* in, T* out) {
-        with_async_kernel<T, 1, false>(lpr, [&](auto kernel) {
-            const int64_t grid = std::min<int64_t>(async_need, async_resident_blocks(kernel));
-            kernel<<<grid, kAsyncBlock, 0, cs>>>(n, rp, ci, v, in, 1, out, 1, nullptr,
-                                                 nullptr, &ctl->all_stopped);
+    auto async_spmv = [&](cudaStream_t cs, const T* in, T* out, const T* a, auto ns) {
+        using Epi = BicgDotEpilogue<T, decltype(ns)::value>;
+        const Epi epi{a, partials, ctl, sc};
+        with_async_epi_kernel<T, Epi>(lpr, [&](auto kernel) {
+            const int64_t grid = std::min<int64_t>(
+                std::min<int64_t>(async_need, async_resident_blocks(kernel)), kSolverGrid);
+            kernel<<<grid, kAsyncBlock, 0, cs>>>(n, rp, ci, v, in, out, &ctl->all_stopped, epi);
         });
     };
+    const std::integral_constant<int, 1> alpha_dot{};
+    const std::integral_constant<int, 3> omega_dots{};
     const bool split = K == 1 && n >= kBicgSplitRows;
     // the split passes with K columns: block Jacobi (any K), and four or
     // more right-hand sides (forming p' and s at every gathered column
@@ -1035,8 +1060,28 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
     // 16-byte column slices where K allows, else the pipelined kernel
     auto split_k_iteration = [&](cudaStream_t cs, int o, int nw) {
         B2S_DISPATCH_RHS(K, {
-            auto spmv_k = [&](const T* in, T* out) {
+            // out = A in and the dots with a (BicgDotEpilogue's)
+            auto spmv_k = [&](const T* in, T* out, const T* a, auto ns) {
+                constexpr int NS = decltype(ns)::value;
                 if constexpr (K >= 4 && K % Vec16<T>::width == 0) {
+                    constexpr int KL = K / Vec16<T>::width;
+                    if (max_row_nnz >= 1 && max_row_nnz <= kRowsMaxLen) {
+                        // rows per warp as in CG's split iteration
+                        auto fused = [&](auto rc) {
+                            constexpr int ROWS = decltype(rc)::value;
+                            auto kernel = bicg_spmv_rows_kernel<T, K, ROWS, NS>;
+                            const int64_t gs = std::min<int64_t>(
+                                ceildiv(ceildiv(n, ROWS), kSolverBlock / kWarp), kSolverGrid);
+                            kernel<<<pgrid(kernel, gs), kSolverBlock, 0, cs>>>(
+                                n, rp, ci, v, in, out, a, ctl, sc, partials);
+                        };
+                        if (KL < 8 && (KL == 1 || max_row_nnz <= kRowsShort)) {
+                            fused(std::integral_constant<int, KL < 8 ? 32 : 16>());
+                        } else {
+                            fused(std::integral_constant<int, KL == 1 ? 32 : 16>());
+                        }
+                        return;
+                    }
                     launch_rhs_lanes<T, K, 0>(n, rp, 0, 0, nullptr, nullptr, ci, v, in, K, out,
                                               K, nullptr, nullptr, max_row_nnz, cs,
                                               &ctl->all_stopped);
@@ -1048,6 +1093,19 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
                                                              nullptr, nullptr,
                                                              &ctl->all_stopped);
                     });
+                }
+                if constexpr (K >= 4 && K % Vec16<T>::width == 0) {
+                    const int gl = int(std::min<int64_t>(
+                        std::max<int64_t>(1, ceildiv(n * K / Vec16<T>::width, kSolverBlock)),
+                        solver_grid()));
+                    bicg_dots_lanes_kernel<T, K, NS><<<pgrid(bicg_dots_lanes_kernel<T, K, NS>, gl), kSolverBlock, 0, cs>>>(
+                        n, a, out, ctl, sc, partials);
+                } else if constexpr (NS == 1) {
+                    bicg_dot1k_kernel<T, K><<<pgrid(bicg_dot1k_kernel<T, K>, grid_vec), kSolverBlock, 0, cs>>>(
+                        n, a, out, ctl, sc, partials);
+                } else {
+                    bicg_dot2k_kernel<T, K><<<pgrid(bicg_dot2k_kernel<T, K>, grid_vec), kSolverBlock, 0, cs>>>(
+                        n, a, out, ctl, sc, partials);
                 }
             };
             constexpr bool kLanes = K >= 4 && K % Vec16<T>::width == 0;
@@ -1064,14 +1122,7 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
                 bicg_vec_k_kernel<T, K, 1><<<pgrid(bicg_vec_k_kernel<T, K, 1>, grid_vec), kSolverBlock, 0, cs>>>(
                     n, dinv, r, p[o], vv[o], p[nw], yv, ctl, sc);
             }
-            spmv_k(yv, vv[nw]);
-            if constexpr (kLanes) {
-                bicg_dots_lanes_kernel<T, K, 1><<<pgrid(bicg_dots_lanes_kernel<T, K, 1>, grid_lanes), kSolverBlock, 0, cs>>>(
-                    n, rr, vv[nw], ctl, sc, partials);
-            } else {
-                bicg_dot1k_kernel<T, K><<<pgrid(bicg_dot1k_kernel<T, K>, grid_vec), kSolverBlock, 0, cs>>>(n, rr, vv[nw], ctl,
-                                                                          sc, partials);
-            }
+            spmv_k(yv, vv[nw], rr, alpha_dot);
             if (bp) {
                 launch_bicg_block_vec<T, K, 2>(n, *bp, r, vv[nw], nullptr, s, zv, ctl, sc, cs);
             } else if constexpr (kLanes) {
@@ -1081,15 +1132,11 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
                 bicg_vec_k_kernel<T, K, 2><<<pgrid(bicg_vec_k_kernel<T, K, 2>, grid_vec), kSolverBlock, 0, cs>>>(
                     n, dinv, r, vv[nw], nullptr, s, zv, ctl, sc);
             }
-            spmv_k(zv, t);
+            spmv_k(zv, t, s, omega_dots);
             if constexpr (kLanes) {
-                bicg_dots_lanes_kernel<T, K, 3><<<pgrid(bicg_dots_lanes_kernel<T, K, 3>, grid_lanes), kSolverBlock, 0, cs>>>(
-                    n, s, t, ctl, sc, partials);
                 bicg_update_lanes_kernel<T, K><<<pgrid(bicg_update_lanes_kernel<T, K>, grid_lanes), kSolverBlock, 0, cs>>>(
                     n, x, ldx, r, rr, yv, s, t, zv, ctl, sc, partials);
             } else {
-                bicg_dot2k_kernel<T, K><<<pgrid(bicg_dot2k_kernel<T, K>, grid_vec), kSolverBlock, 0, cs>>>(n, s, t, ctl, sc,
-                                                                          partials);
                 bicg_update_kernel<T, K><<<pgrid(bicg_update_kernel<T, K>, grid_vec), kSolverBlock, 0, cs>>>(
                     n, nullptr, x, ldx, r, rr, yv, s, t, ctl, sc, partials, zv);
             }
@@ -1107,14 +1154,10 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
             if (split) {
                 bicg_pupdate_kernel<T><<<pgrid(bicg_pupdate_kernel<T>, grid_vec), kSolverBlock, 0, cs>>>(
                     n, dinv, r, p[o], vv[o], p[nw], yv, ctl, sc);
-                async_spmv(cs, yv, vv[nw]);
-                bicg_dot1_kernel<T><<<pgrid(bicg_dot1_kernel<T>, grid_vec), kSolverBlock, 0, cs>>>(n, rr, vv[nw], ctl, sc,
-                                                                      partials);
+                async_spmv(cs, yv, vv[nw], rr, alpha_dot);
                 bicg_supdate_kernel<T><<<pgrid(bicg_supdate_kernel<T>, grid_vec), kSolverBlock, 0, cs>>>(
                     n, dinv, r, vv[nw], s, zv, ctl, sc);
-                async_spmv(cs, zv, t);
-                bicg_dot2_kernel<T><<<pgrid(bicg_dot2_kernel<T>, grid_vec), kSolverBlock, 0, cs>>>(n, s, t, ctl, sc,
-                                                                      partials);
+                async_spmv(cs, zv, t, s, omega_dots);
                 bicg_update_kernel<T, 1><<<pgrid(bicg_update_kernel<T, 1>, grid_vec), kSolverBlock, 0, cs>>>(
                     n, dinv, x, ldx, r, rr, p[nw], s, t, ctl, sc, partials);
                 B2S_LAUNCH_CHECK();

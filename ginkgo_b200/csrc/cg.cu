@@ -53,53 +53,6 @@ __device__ __forceinline__ T cg_p(T d, T r, T beta, T p, bool from_z)
     return from_z ? z : add_rn(z, mul_rn(beta, p));
 }
 
-// tot[a * K + j] = sum over blocks of partials[(a * nblocks + b) * K + j],
-// a < A: thread t takes value t % K of blocks t / K, t / K + 256 / K, ... (the
-// loads of a warp are consecutive and eight are in flight), then the slots
-// are added in order.  Deterministic for a fixed grid.  Out of line: its
-// loads in flight would set the register count of the whole pass.
-// sum_partials has every thread walk all K values of its blocks, 16 loads and
-// 80 shuffles deep with 16 columns.
-template <typename T, int K, int A>
-__device__ __noinline__ void cg_fold(const T* partials, int nblocks, T* tot)
-{
-    constexpr int kSlots = kSolverBlock / K;
-    __shared__ T sm[A][kSolverBlock];
-    const int j = threadIdx.x % K, slot = threadIdx.x / K;
-    T acc[A];
-#pragma unroll
-    for (int a = 0; a < A; ++a) acc[a] = T(0);
-    for (int b0 = slot; b0 < nblocks; b0 += 8 * kSlots) {
-        T v[A][8];
-#pragma unroll
-        for (int a = 0; a < A; ++a) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int b = b0 + q * kSlots;
-                v[a][q] = b < nblocks ? __ldcg(partials + (int64_t(a) * nblocks + b) * K + j) : T(0);
-            }
-        }
-#pragma unroll
-        for (int a = 0; a < A; ++a) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q) acc[a] += v[a][q];
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < A; ++a) sm[a][threadIdx.x] = acc[a];
-    __syncthreads();
-#pragma unroll
-    for (int half = kSlots / 2; half > 0; half /= 2) {
-        if (slot < half) {
-#pragma unroll
-            for (int a = 0; a < A; ++a) sm[a][threadIdx.x] += sm[a][threadIdx.x + half * K];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x < A * K) tot[threadIdx.x] = sm[threadIdx.x / K][threadIdx.x % K];
-    __syncthreads();
-}
-
 // The last block's part of the initial pass (its first warp, lane j taking
 // column j): tot holds ||b||^2, rho = dot(r, z) and ||r||^2 of every column
 // (K each); sets the starting norms, rho and the initial stopping status.
@@ -410,7 +363,7 @@ __global__ void __launch_bounds__(kSolverBlock)
         partials[blockIdx.x * K + threadIdx.x] = s;
     }
     if (last_block_done(&ctl->ticket, &last)) {
-        cg_fold<T, K, 1>(partials, gridDim.x, tot);
+        fold_columns<T, K, 1>(partials, gridDim.x, tot);
         if (threadIdx.x < K) {
             const T pq = tot[threadIdx.x];
             sc->alpha[threadIdx.x] = pq != T(0) ? sc->rho[threadIdx.x] / pq : T(0);
@@ -491,7 +444,7 @@ __global__ void __launch_bounds__(kSolverBlock)
         partials[(threadIdx.x < K ? 0 : int64_t(gridDim.x) * K) + blockIdx.x * K + j] = s;
     }
     if (last_block_done(&ctl->ticket, &last)) {
-        cg_fold<T, K, 2>(partials, gridDim.x, tot);
+        fold_columns<T, K, 2>(partials, gridDim.x, tot);
         if (threadIdx.x < kWarp) cg_update_finish<T, K>(tot, ctl, sc);
     }
 }
@@ -725,7 +678,7 @@ __global__ void __launch_bounds__(kSolverBlock)
         partials[blockIdx.x * K + threadIdx.x] = s;
     }
     if (last_block_done(&ctl->ticket, &last)) {
-        cg_fold<T, K, 1>(partials, gridDim.x, tot);
+        fold_columns<T, K, 1>(partials, gridDim.x, tot);
         if (threadIdx.x < K) cg_alpha(threadIdx.x, tot[threadIdx.x], ctl, sc);
         if (threadIdx.x == 0) ctl->ticket = 0;
     }
@@ -810,7 +763,7 @@ __global__ void __launch_bounds__(kSolverBlock)
         partials[(threadIdx.x < K ? 0 : int64_t(gridDim.x) * K) + blockIdx.x * K + j] = s;
     }
     if (last_block_done(&ctl->ticket, &last)) {
-        cg_fold<T, K, 2>(partials, gridDim.x, tot);
+        fold_columns<T, K, 2>(partials, gridDim.x, tot);
         if (threadIdx.x < kWarp) cg_update_finish<T, K>(tot, ctl, sc);
     }
 }

@@ -205,6 +205,53 @@ __device__ __forceinline__ void sum_partials(const T* partials, int nblocks,
     __syncthreads();
 }
 
+// tot[a * K + j] = sum over blocks of partials[(a * nblocks + b) * K + j],
+// a < A: thread t takes value t % K of blocks t / K, t / K + 256 / K, ... (the
+// loads of a warp are consecutive and eight are in flight), then the slots
+// are added in order.  Deterministic for a fixed grid.  Out of line: its
+// loads in flight would set the register count of the whole pass.
+// sum_partials has every thread walk all K values of its blocks, 16 loads and
+// 80 shuffles deep with 16 columns.
+template <typename T, int K, int A>
+__device__ __noinline__ void fold_columns(const T* partials, int nblocks, T* tot)
+{
+    constexpr int kSlots = kSolverBlock / K;
+    __shared__ T sm[A][kSolverBlock];
+    const int j = threadIdx.x % K, slot = threadIdx.x / K;
+    T acc[A];
+#pragma unroll
+    for (int a = 0; a < A; ++a) acc[a] = T(0);
+    for (int b0 = slot; b0 < nblocks; b0 += 8 * kSlots) {
+        T v[A][8];
+#pragma unroll
+        for (int a = 0; a < A; ++a) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int b = b0 + q * kSlots;
+                v[a][q] = b < nblocks ? __ldcg(partials + (int64_t(a) * nblocks + b) * K + j) : T(0);
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < A; ++a) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[a] += v[a][q];
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < A; ++a) sm[a][threadIdx.x] = acc[a];
+    __syncthreads();
+#pragma unroll
+    for (int half = kSlots / 2; half > 0; half /= 2) {
+        if (slot < half) {
+#pragma unroll
+            for (int a = 0; a < A; ++a) sm[a][threadIdx.x] += sm[a][threadIdx.x + half * K];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x < A * K) tot[threadIdx.x] = sm[threadIdx.x / K][threadIdx.x % K];
+    __syncthreads();
+}
+
 // r = b - A x for the first k of K columns (the rest zero); b, x strided,
 // r contiguous n x K.  One subwarp of SW lanes per row, grid-stride.
 template <typename T, int SW, int K>
