@@ -316,20 +316,12 @@ __device__ __forceinline__ int dots_row(int c, int nvec)
     return c < nvec ? c : kLd + c - nvec;
 }
 
-// Ticket of `count` arrivals; true in the last one to arrive (the caller's
-// writes are fenced first), which resets the ticket.
+// Ticket of `count` arrivals; true in the last one to arrive, which resets
+// the ticket.
 __device__ __forceinline__ bool last_of(unsigned* ticket, unsigned count, int* flag_sm)
 {
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned t = atomicAdd(ticket, 1u);
-        *flag_sm = (t == count - 1);
-        if (t == count - 1) *ticket = 0;
-    }
-    __syncthreads();
-    const bool last = *flag_sm;
-    if (last) __threadfence();
+    const bool last = arrive_ticket(ticket, flag_sm) == count - 1;
+    if (last && threadIdx.x == 0) *ticket = 0;
     return last;
 }
 
@@ -382,11 +374,21 @@ __global__ void __launch_bounds__(kSolverBlock, 4)
     __shared__ double redv[W][8];
     __shared__ double tot[2 * kLd];
     __shared__ double Gs[kSmallGram * kSmallGram];
+    __shared__ double sig[kLd];
     __shared__ int last;
-    if (st->idle) return;
-    const int j = st->j;
+    // the state, in one round of loads
+    const int idle = st->idle, j = st->j, ortho = st->ortho, ld = st->ld;
+    if (idle) return;
     const int nvec = j + 1;
     const int lane = threadIdx.x % kWarp, wid = threadIdx.x / kWarp;
+    // what the last block will need of the earlier steps, while the basis
+    // streams in: the scales, and G(i, k), i, k < j (short cycles)
+    for (int i = threadIdx.x; i < nvec; i += kSolverBlock) sig[i] = st->sigma[i];
+    if (j < kSmallGram && ortho != B2S_ORTHO_CGS) {
+        for (int i = wid; i < j; i += W) {
+            if (lane < j) Gs[i * kSmallGram + lane] = Gm[int64_t(i) * ld + lane];
+        }
+    }
     const TB* vj = V + int64_t(j) * ldv;
     const int B = gridDim.x;
     for (int i0 = 0; i0 < nvec; i0 += CMAX) {
@@ -427,27 +429,22 @@ __global__ void __launch_bounds__(kSolverBlock, 4)
     fold32(gpart, kDotsMaxGroups, 0, ngroups, nvec, tot, 1, 0);
     __syncthreads();
     if (threadIdx.x <= j) {
-        const double sc = st->sigma[threadIdx.x] * st->sigma[j];
+        const double sc = sig[threadIdx.x] * sig[j];
         tot[threadIdx.x] *= sc;
         tot[kLd + threadIdx.x] *= sc;
     }
     __syncthreads();
-    if (st->ortho == B2S_ORTHO_CGS) {
+    if (ortho == B2S_ORTHO_CGS) {
         // one projection: h = h1
         if (threadIdx.x <= j) st->h[threadIdx.x] = tot[threadIdx.x];
         return;
     }
     // row and column j of G; rows 0..j-1 hold the earlier steps of this
     // cycle (G is symmetric, so row i of G(0..j, 0..j) is complete)
-    const int ld = st->ld;
     if (j < kSmallGram) {
-        // the whole G(0..j, 0..j) in shared memory (one parallel pass of
-        // loads), then one thread per row: the short serial tail of every
-        // Arnoldi step of the usual Krylov dimensions
-        for (int e = threadIdx.x; e < j * j; e += kSolverBlock) {
-            const int i = e / j, k = e - i * j;  // G(i, k), i, k < j: earlier steps
-            Gs[i * kSmallGram + k] = __ldcg(Gm + int64_t(i) * ld + k);
-        }
+        // the whole G(0..j, 0..j) in shared memory, then one thread per row:
+        // the short serial tail of every Arnoldi step of the usual Krylov
+        // dimensions
         if (threadIdx.x <= j) {  // row and column j: this step
             const int i = threadIdx.x;
             const double gij = tot[kLd + i];
@@ -460,6 +457,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4)
         if (threadIdx.x <= j) {
             const int i = threadIdx.x;
             double gh = 0.0;
+#pragma unroll 8
             for (int k = 0; k <= j; ++k) gh += Gs[i * kSmallGram + k] * tot[k];
             st->h[i] = 2.0 * tot[i] - gh;
         }
@@ -482,36 +480,50 @@ __global__ void __launch_bounds__(kSolverBlock, 4)
     }
 }
 
+// What the end of Arnoldi step j reads of the state, loaded by every block of
+// the update pass while the basis streams in, so that the last block's serial
+// tail does not wait for it.
+struct StepState {
+    double hc[kLd], g[kLd], cs[kMaxKrylov], sn[kMaxKrylov];
+    double inner_thresh;
+    int total_iter, max_iters, krylov_dim, ld;
+};
+
 // The end of Arnoldi step j, run by the whole last block of the update
 // kernel: Givens update of column j, residual estimate, cycle bookkeeping
 // and, when the cycle ends, the back substitution y = H \ g.  The small
 // arrays are staged in shared memory, so the serial chain runs at
-// shared-memory latency.
-__device__ __noinline__ void close_step(GmresState* st, double hnorm, double* __restrict__ Hm)
+// shared-memory latency, eight rotations' operands loaded ahead of their
+// chain of one multiply-add each.
+__device__ __noinline__ void close_step(GmresState* st, int j, double hnorm, StepState* ss,
+                                        double* __restrict__ Hm)
 {
-    __shared__ double hc[kLd], gS[kLd], csS[kMaxKrylov], snS[kMaxKrylov];
     __shared__ double ts[kMaxKrylov];
     __shared__ int fin;
-    const int j = st->j;
-    const int ld = st->ld;
-    for (int i = threadIdx.x; i <= j; i += kSolverBlock) {
-        hc[i] = st->h[i];
-        gS[i] = st->g[i];
-    }
-    for (int i = threadIdx.x; i < j; i += kSolverBlock) {
-        csS[i] = st->cs[i];
-        snS[i] = st->sn[i];
-    }
-    __syncthreads();
+    double* hc = ss->hc;
+    double* gS = ss->g;
+    const int ld = ss->ld;
     if (threadIdx.x == 0) {
         st->ticket = 0;
-        hc[j + 1] = hnorm;
-        for (int i = 0; i < j; ++i) {
-            const double t = csS[i] * hc[i] + snS[i] * hc[i + 1];
-            hc[i + 1] = -snS[i] * hc[i] + csS[i] * hc[i + 1];
-            hc[i] = t;
+        double carry = hc[0];  // row i of the column, rotated so far
+        for (int i0 = 0; i0 < j; i0 += 8) {
+            double c8[8], s8[8], h8[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const bool in = i0 + u < j;
+                c8[u] = in ? ss->cs[i0 + u] : 1.0;
+                s8[u] = in ? ss->sn[i0 + u] : 0.0;
+                h8[u] = in ? hc[i0 + u + 1] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (i0 + u < j) {
+                    hc[i0 + u] = c8[u] * carry + s8[u] * h8[u];
+                    carry = -s8[u] * carry + c8[u] * h8[u];
+                }
+            }
         }
-        const double th = hc[j], nh = hc[j + 1];
+        const double th = carry, nh = hnorm;
         double c, s;
         if (th == 0.0) {
             c = 0.0;
@@ -523,22 +535,23 @@ __device__ __noinline__ void close_step(GmresState* st, double hnorm, double* __
             c = th / hyp;
             s = nh / hyp;
         }
+        const double gj = gS[j];
         hc[j] = c * th + s * nh;
         hc[j + 1] = 0.0;
-        gS[j + 1] = -s * gS[j];
-        gS[j] = c * gS[j];
+        gS[j + 1] = -s * gj;
+        gS[j] = c * gj;
         st->cs[j] = c;
         st->sn[j] = s;
-        st->g[j] = gS[j];
-        st->g[j + 1] = gS[j + 1];
-        const double est = fabs(gS[j + 1]);
-        const int total = st->total_iter + 1;
+        st->g[j] = c * gj;
+        st->g[j + 1] = -s * gj;
+        const double est = fabs(s * gj);
+        const int total = ss->total_iter + 1;
         st->final_iter = j + 1;
         st->total_iter = total;
         st->sigma[j + 1] = hnorm > 0.0 ? 1.0 / hnorm : 0.0;
         st->j = j + 1;
-        fin = est <= st->inner_thresh || j + 1 >= st->krylov_dim ||
-              total >= st->max_iters || !(hnorm > 0.0);
+        fin = est <= ss->inner_thresh || j + 1 >= ss->krylov_dim ||
+              total >= ss->max_iters || !(hnorm > 0.0);
         if (fin) {
             st->cycle_done = 1;
             st->idle = 1;
@@ -606,10 +619,27 @@ __global__ void __launch_bounds__(kSolverBlock, (update_min_blocks<TA, TB>()))
     __shared__ double red[kSolverBlock / kWarp];
     __shared__ double tot[1];
     __shared__ TA hs[kLd];
+    __shared__ StepState ss;
     __shared__ int last;
-    if (st->idle) return;
-    const int j = st->j;
-    for (int i = threadIdx.x; i <= j; i += kSolverBlock) hs[i] = TA(st->h[i] * st->sigma[i]);
+    const int idle = st->idle, j = st->j;
+    if (idle) return;
+    for (int i = threadIdx.x; i <= j; i += kSolverBlock) {
+        const double h = st->h[i];
+        hs[i] = TA(h * st->sigma[i]);
+        ss.hc[i] = h;
+        ss.g[i] = st->g[i];
+        if (i < j) {
+            ss.cs[i] = st->cs[i];
+            ss.sn[i] = st->sn[i];
+        }
+    }
+    if (threadIdx.x == kSolverBlock - 1) {
+        ss.inner_thresh = st->inner_thresh;
+        ss.total_iter = st->total_iter;
+        ss.max_iters = st->max_iters;
+        ss.krylov_dim = st->krylov_dim;
+        ss.ld = st->ld;
+    }
     const TA sj = TA(st->sigma[j]);
     __syncthreads();
     TB* vnext = V + int64_t(j + 1) * ldv;
@@ -675,7 +705,7 @@ __global__ void __launch_bounds__(kSolverBlock, (update_min_blocks<TA, TB>()))
     if (last_block_done(&st->ticket, &last)) {
         sum_partials<double, 1>(partials, gridDim.x, tot, red);
         const double hnorm = sqrt(tot[0]);
-        close_step(st, hnorm, Hm);
+        close_step(st, j, hnorm, &ss, Hm);
         if constexpr (kQ) {
             if (threadIdx.x == 0) {
                 double m = 0.0;

@@ -143,19 +143,27 @@ __device__ __forceinline__ void block_partials(T (&v)[K], T* __restrict__ partia
     }
 }
 
+// Counts the calling block in on `ticket` and returns (to every thread) the
+// arrivals before it.  The block's writes are released and, for the last
+// arrival, the others' acquired by one thread: the block barriers order the
+// rest of the block around its fences (a sequentially consistent fence in
+// every thread instead cost about a microsecond of each reduction's tail).
+__device__ __forceinline__ unsigned arrive_ticket(unsigned* ticket, int* flag_sm)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        *flag_sm = int(atomicAdd(ticket, 1u));
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    }
+    __syncthreads();
+    return unsigned(*flag_sm);
+}
+
 // True in exactly one block: the last one to finish its partials.
 __device__ __forceinline__ bool last_block_done(unsigned* ticket, int* flag_sm)
 {
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned t = atomicAdd(ticket, 1u);
-        *flag_sm = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    const bool last = *flag_sm;
-    if (last) __threadfence();
-    return last;
+    return arrive_ticket(ticket, flag_sm) == gridDim.x - 1;
 }
 
 // In the last block: out[j] = sum over blocks of partials[b][j], summed in a
