@@ -30,9 +30,10 @@
 //
 // Kernels per Arnoldi step j (one CUDA graph per restart cycle):
 //   spmv    w = A y on a column-major (Ell) copy of A in the Arnoldi type
-//           with 16-bit column offsets (32-bit columns when an offset does
-//           not fit), when its padding stays within a quarter of nnz; else
-//           the pipelined Csr kernel on A
+//           when its padding stays within a quarter of nnz, with column
+//           offsets shared by 32 rows where they fit the width, else 16-bit
+//           offsets (32-bit columns when an offset does not fit); else the
+//           pipelined Csr kernel on A
 //   dots    h1 = V_{0..j}^T w and G(:, j) = V_{0..j}^T v_j in one pass over
 //           the basis (all sums of a thread in registers); last block:
 //           h = (2I - G) h1
@@ -76,6 +77,7 @@ struct GmresState {
     unsigned ticket;
     int too_long;  // a row is longer than the Ell copy's width
     int too_far;   // a column offset does not fit 16 bits
+    int too_wide;  // 32 rows have more column offsets than the copy's width
     unsigned gticket[kDotsMaxGroups + 1];  // dots: per group of 32 blocks
     double bnorm, rnorm, reduction, inner_reduction, inner_thresh;
     double base;  // ||b||, ||r_0|| or 1, by the baseline, set at the first restart
@@ -1133,7 +1135,25 @@ int gmres_engine(const GmresLayout& lay, int64_t n, int64_t nnz, const int32_t* 
     TA* ell_v = reinterpret_cast<TA*>(w + lay.off_ell_v);
     // 16-bit column offsets when every |col - row| fits, else 32-bit columns
     bool ell16 = false;
-    if (ell_w > 0) {
+    // offsets shared by 32 rows where the width allows (stencils): 27-point
+    // 96^3 in FP64 48.3 -> 37.1 us per product (200 MB in place of 253 MB, at
+    // 0.89 of the copy rate).  In FP32 up to 2^19 rows, where the Ell form's
+    // four rows per thread leave too few threads (IR, Krylov dimension 30, 360
+    // iterations: 24^3 11.0 -> 9.3 ms, 64^3 16.7 -> 13.2 ms); on 96^3 both
+    // take 30 us.
+    constexpr int64_t kSliceRowsF32 = int64_t(1) << 19;
+    bool sliced = false;
+    if (ell_w > 0 && (sizeof(TA) == 8 || n <= kSliceRowsF32)) {
+        slice_fill_kernel<TA><<<ceildiv(ldv, 256), 256, 0, st>>>(n, ell_w, rp, ci, v64, ell_c,
+                                                                 ell_v, &gs->too_wide);
+        B2S_LAUNCH_CHECK();
+        int wide = 0;
+        B2S_CUDA_TRY(cudaMemcpyAsync(&wide, &gs->too_wide, sizeof(wide), cudaMemcpyDeviceToHost,
+                                     st));
+        B2S_CUDA_TRY(cudaStreamSynchronize(st));
+        sliced = !wide;
+    }
+    if (ell_w > 0 && !sliced) {
         ell_fill16_kernel<TA><<<ceildiv(ldv, 256), 256, 0, st>>>(
             n, ldv, ell_w, rp, ci, v64, reinterpret_cast<int16_t*>(ell_c), ell_v,
             &gs->too_long, &gs->too_far);
@@ -1212,7 +1232,11 @@ int gmres_engine(const GmresLayout& lay, int64_t n, int64_t nnz, const int32_t* 
             // y (the SpMV input) was written by the restart kernel (j = 0)
             // or by the previous step's update
             TA* dst = wbuf;
-            if (ell_w > 0) {
+            if (sliced) {
+                auto kernel = slice_rows_kernel<TA>;
+                kernel<<<pgrid(kernel, std::max<int64_t>(1, ceildiv(n, 256))), 256, 0, cs>>>(
+                    n, ell_w, ell_c, ell_v, y, dst, &gs->idle);
+            } else if (ell_w > 0) {
                 const int16_t* c16 = reinterpret_cast<const int16_t*>(ell_c);
                 if (ell_r == kEllRows && ell16) {
                     ell_rows_kernel_for<TA, kEllRows, true, int16_t>()<<<grid_ell, 256, 0, cs>>>(
