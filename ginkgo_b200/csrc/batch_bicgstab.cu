@@ -189,7 +189,8 @@ __global__ void __launch_bounds__(kBatchBlock, batch_min_blocks<T, RPT>())
         if (q >= a.num_sys) break;  // whole group
         const int sys = a.sys_list[q];
         const int off = a.uniform_n ? sys * a.uniform_n : a.row_offsets[sys];
-        const int n = a.uniform_n ? a.uniform_n : a.row_offsets[sys + 1] - off;
+        int n = a.uniform_n ? a.uniform_n : a.row_offsets[sys + 1] - off;
+        if constexpr (kStage) n = n < a.nstage ? n : a.nstage;  // the stage's rows
         const int64_t vbase = int64_t(a.width) * off;
         const int32_t* cs = a.uniform_n ? ci : ci + vbase;
         const T* vs = val + vbase;

@@ -777,17 +777,21 @@ __global__ void __launch_bounds__(kSolverBlock)
 // threads) owns RPT rows and keeps their r, x, p, q and D^-1 in registers;
 // r and p go to global memory only for the other rows' gathers, which read
 // L2 (__ldcg), p double buffered as in the fused passes.
-// 5-point 256^2 to 1e-10 (710 iterations): 11.3 -> 6.0 ms.
+// 5-point 256^2 to 1e-10 (710 iterations): 11.7 -> 5.8 ms.
 // ---------------------------------------------------------------------------
 constexpr int kCgResidentBlock = 512;
 constexpr int kCgResidentIters = 1 << 13;  // iterations per launch
+// Status of the loop when the device cannot hold its blocks at once (a
+// limited share of the SMs) or a block's entries exceed its stage (rows
+// longer than max_row_nnz): nothing has run, the passes take the solve.
+constexpr int kCgNotResident = 1;
 
 template <typename T, int SW, int RPT>
 __global__ void __launch_bounds__(kCgResidentBlock, 1)
     cg_resident_kernel(int64_t n, const int32_t* __restrict__ rp,
                        const int32_t* __restrict__ ci, const T* __restrict__ v,
                        const T* __restrict__ dinv, T* __restrict__ x, int64_t ldx, T* r, T* p0,
-                       T* p1, SolveCtl* ctl, CgScalars<T>* sc, ExchangeSlot* slots)
+                       T* p1, SolveCtl* ctl, CgScalars<T>* sc, ExchangeSlot* slots, int capacity)
 {
     extern __shared__ __align__(16) unsigned char stage_raw[];
     __shared__ double red[kExchangeShared];
@@ -820,7 +824,19 @@ __global__ void __launch_bounds__(kCgResidentBlock, 1)
     // they would come from L2 in every iteration)
     const int e0 = rp[row0], cnt = rp[row1] - e0;
     T* mv = reinterpret_cast<T*>(stage_raw);
-    int32_t* mc = reinterpret_cast<int32_t*>(mv + cnt);
+    int32_t* mc = reinterpret_cast<int32_t*>(mv + capacity);
+    unsigned epoch = 0;
+    // rows longer than the caller said: all blocks leave together, nothing
+    // written
+    T over[1] = {threadIdx.x == 0 && cnt > capacity ? T(1) : T(0)};
+    if (!grid_exchange<T, 1>(over, slots, ++epoch, red)) {
+        if (threadIdx.x == 0) ctl->failed = 1;
+        return;
+    }
+    if (over[0] != T(0)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->failed = 2;
+        return;
+    }
     for (int e = threadIdx.x; e < cnt; e += kCgResidentBlock) {
         mv[e] = v[e0 + e];
         mc[e] = ci[e0 + e];
@@ -839,7 +855,6 @@ __global__ void __launch_bounds__(kCgResidentBlock, 1)
     uint8_t status = ctl->status[0];
     T rho = sc->rho[0], prev_rho = sc->prev_rho[0], tau = sc->tau[0];
     const T start = sc->start[0];
-    unsigned epoch = 0;
     while (!has_stopped(status) && iter < last) {
         const bool from_z = prev_rho == T(0);
         const T beta = from_z ? T(0) : rho / prev_rho;
@@ -953,15 +968,23 @@ int cg_resident_loop(int64_t n, const int32_t* rp, const int32_t* ci, const T* v
     const size_t smem = size_t(need);
     B2S_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       int(kCgStageBytes)));
-    void* args[] = {&n, &rp, &ci, &v, &dinv, &x, &ldx, &r, &p0, &p1, &ctl, &sc, &slots};
+    int capacity = int(need / int64_t(sizeof(T) + 4));  // entries of a block's stage
+    void* args[] = {&n,  &rp, &ci,  &v,  &dinv,  &x,       &ldx, &r,
+                    &p0, &p1, &ctl, &sc, &slots, &capacity};
     const int64_t max_launches = int64_t(max_iters) / kCgResidentIters + 2;
     for (int64_t l = 0; l < max_launches; ++l) {
         B2S_CUDA_TRY(cudaMemsetAsync(slots, 0, kExchangeSlots * sizeof(ExchangeSlot), st));
-        B2S_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel),
-                                                 dim3(unsigned(grid)), dim3(kCgResidentBlock),
-                                                 args, smem, st));
+        const cudaError_t e = cudaLaunchCooperativeKernel(
+            reinterpret_cast<const void*>(kernel), dim3(unsigned(grid)), dim3(kCgResidentBlock),
+            args, smem, st);
+        if (e != cudaSuccess && l == 0) {
+            (void)cudaGetLastError();
+            return kCgNotResident;
+        }
+        B2S_CUDA_TRY(e);
         B2S_CUDA_TRY(cudaMemcpyAsync(host_ctl, ctl, sizeof(SolveCtl), cudaMemcpyDeviceToHost, st));
         B2S_CUDA_TRY(cudaStreamSynchronize(st));
+        if (host_ctl->failed == 2) return kCgNotResident;
         if (host_ctl->failed) {
             set_error("CG: the blocks of the resident kernel did not meet");
             return B2S_ERR_CUDA;
@@ -1321,12 +1344,15 @@ int cg_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
     };
     // the graph always runs an even number of iterations, so p[0] holds the
     // current direction at every replay boundary
-    const bool resident = K == 1 && !bp && cg_resident_ok<T>(n, max_row_nnz);
-    int rc = resident
-                 ? cg_resident_loop<T>(n, rp, ci, v, dinv, x, ldx, r, p[0], p[1], ctl, sc,
-                                       reinterpret_cast<ExchangeSlot*>(w + lay.off_slots),
-                                       max_row_nnz, int(max_iters), st, &h)
-                 : run_graph_loop(st, ctl, int(max_iters), chunk, capture, &h);
+    bool resident = K == 1 && !bp && cg_resident_ok<T>(n, max_row_nnz);
+    int rc = B2S_OK;
+    if (resident) {
+        rc = cg_resident_loop<T>(n, rp, ci, v, dinv, x, ldx, r, p[0], p[1], ctl, sc,
+                                 reinterpret_cast<ExchangeSlot*>(w + lay.off_slots),
+                                 max_row_nnz, int(max_iters), st, &h);
+        resident = rc != kCgNotResident;
+    }
+    if (!resident) rc = run_graph_loop(st, ctl, int(max_iters), chunk, capture, &h);
     if (rc != B2S_OK) return rc;
     if (split && !bp && !resident) {
         B2S_DISPATCH_RHS(K, {

@@ -43,7 +43,10 @@ class CudaExecutor:
 
 def _stream(t: torch.Tensor):
     # the handle alone: a torch.cuda.Stream object costs about 1.5 us
-    return torch._C._cuda_getCurrentRawStream(t.device.index)
+    index = t.device.index
+    if index is None:  # not a CUDA tensor: raises
+        return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(index)
 
 
 def _p(t):

@@ -102,3 +102,18 @@ def test_columns_stop_apart(n, band, k, its):
         ref, _ = cg(rp, ci, v, b[:, j], x0[:, j], its, 1e-12)
         assert np.linalg.norm(got[:, j] - ref) <= 1e-10 * np.linalg.norm(ref), j
     assert bool((wide[:, k] == 7.0).all())
+
+
+@pytest.mark.parametrize("n", [700, 75777])
+def test_rows_longer_than_said(n):
+    """An understated longest row must not size the resident kernel's stage."""
+    exe = CudaExecutor.create(0)
+    rp, ci, v = banded(n, 2, n)
+    b = np.random.default_rng(3).standard_normal(n)
+    A = Csr.read(exe, rp, ci, v)
+    A._max_row_nnz = 1
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    s = solver(exe, A, 200, 1e-12)
+    s.apply(torch.from_numpy(b).cuda(), x)
+    ref, _ = cg(rp, ci, v, b, np.zeros(n), 200, 1e-12)
+    assert np.linalg.norm(x.cpu().numpy() - ref) <= 1e-10 * np.linalg.norm(ref)
