@@ -126,9 +126,11 @@ constexpr int batch_vec_entries()
 // 1024 rows of five FP64 entries), and the group's barriers and reductions
 // need other groups to hide behind (one block per SM at 130 registers: 6.3
 // ms on the workload above).
-template <typename T, int RPT>
+// The forms that read the matrix from global memory are left unconstrained.
+template <typename T, int RPT, int PLACE>
 constexpr int batch_min_blocks()
 {
+    if (PLACE != kSmemAll) return 1;
     return sizeof(T) == 8 ? (RPT <= 4 ? 3 : 1) : (RPT <= 2 ? 4 : RPT <= 4 ? 3 : RPT <= 8 ? 2 : 1);
 }
 
@@ -139,11 +141,13 @@ constexpr int batch_min_blocks()
 // conflict-free shared-memory loads.  8192 FP64 systems of 32 to 1024 rows
 // and five entries per row: 8.7 ms per solve before; 4.5 ms with the stage,
 // the rows' entries loaded side by side and three blocks per SM; 3.06 ms
-// with the overlapped launches below in place of a graph per call.  An entry without a column (padding)
+// with the overlapped launches below in place of a graph per call.  1000 rows
+// of 3 / 9 / 14 / 20 entries (the last two one block per SM): 3.0 / 2.0 / 1.05
+// / 1.1 times as fast as from global memory, which wider systems keep.  An entry without a column (padding)
 // is staged as value 0 with the column of a zero slot past the vector, so
 // the sum needs no test.
 template <typename T, int G, int RPT, int PLACE>
-__global__ void __launch_bounds__(kBatchBlock, batch_min_blocks<T, RPT>())
+__global__ void __launch_bounds__(kBatchBlock, (batch_min_blocks<T, RPT, PLACE>()))
     batch_bicgstab_kernel(BatchArgs a, const int32_t* __restrict__ ci,
                           const T* __restrict__ val, const T* __restrict__ b,
                           T* __restrict__ x, T* __restrict__ gscratch)
@@ -197,24 +201,34 @@ __global__ void __launch_bounds__(kBatchBlock, batch_min_blocks<T, RPT>())
         // r holds s between the two half steps
         T r[RPT], rh[RPT], p[RPT], v[RPT], tt[RPT], xx[RPT], pr[RPT];
         T bb2 = T(0);
-        // acc = A z on the thread's rows: entry j of all its rows at once,
-        // so their load chains (column, then vector) overlap; each row still
-        // sums in entry order
+        // acc = A z on the thread's rows, each row summed in entry order.
+        // Staged: entry j of all the rows at once, so their load chains
+        // (column, then vector) overlap.  From global memory: row by row,
+        // several entries' loads ahead of their sums (entry by entry, the
+        // padding test became a branch per load: 2-3 times as long).
         auto product = [&](T (&acc)[RPT]) {
+            if constexpr (kStage) {
 #pragma unroll
-            for (int k = 0; k < RPT; ++k) acc[k] = T(0);
-            for (int j = 0; j < a.width; ++j) {
+                for (int k = 0; k < RPT; ++k) acc[k] = T(0);
+                for (int j = 0; j < a.width; ++j) {
+#pragma unroll
+                    for (int k = 0; k < RPT; ++k) {
+                        const int row = t + k * G;
+                        if (row < n) acc[k] += mv[row + j * n] * z[mc[row + j * n]];
+                    }
+                }
+            } else {
 #pragma unroll
                 for (int k = 0; k < RPT; ++k) {
                     const int row = t + k * G;
+                    T sum = T(0);
                     if (row < n) {
-                        if constexpr (kStage) {
-                            acc[k] += mv[row + j * n] * z[mc[row + j * n]];
-                        } else {
+                        for (int j = 0; j < a.width; ++j) {
                             const int c = cs[row + j * n];
-                            if (unsigned(c) < unsigned(n)) acc[k] += vs[row + j * n] * z[c];
+                            if (unsigned(c) < unsigned(n)) sum += vs[row + j * n] * z[c];
                         }
                     }
+                    acc[k] = sum;
                 }
             }
         };
