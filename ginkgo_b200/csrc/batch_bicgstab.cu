@@ -142,8 +142,9 @@ constexpr int batch_min_blocks()
 // and five entries per row: 8.7 ms per solve before; 4.5 ms with the stage,
 // the rows' entries loaded side by side and three blocks per SM; 3.06 ms
 // with the overlapped launches below in place of a graph per call.  1000 rows
-// of 3 / 9 / 14 / 20 entries (the last two one block per SM): 3.0 / 2.0 / 1.05
-// / 1.1 times as fast as from global memory, which wider systems keep.  An entry without a column (padding)
+// of 3 / 9 entries: 3.0 / 1.9 times as fast as before.  A block that would
+// leave no room for a second one on its SM keeps the matrix in global memory
+// (400 rows of 20 entries: staged, one block, 2.03 ms; global 1.32 ms).  An entry without a column (padding)
 // is staged as value 0 with the column of a zero slot past the vector, so
 // the sum needs no test.
 template <typename T, int G, int RPT, int PLACE>
@@ -387,8 +388,8 @@ size_t batch_smem_bytes(BatchPlace place, int nstage, int width)
     return bytes;
 }
 
-// Shared memory a block may ask for.
-constexpr size_t kMaxBlockSmem = 227 * 1024;
+// Shared memory of a block that stages its systems: two blocks per SM.
+constexpr size_t kMaxStageSmem = 112 * 1024;
 
 // Launches one configuration of the kernel on a bucket; scratch holds the
 // vectors of kGlobalVecs.  overlap: the kernel may start before the one
@@ -402,7 +403,7 @@ int launch_placed(const BatchArgs& a, const int32_t* ci, const T* val, const T* 
     const size_t sm = batch_smem_bytes<T, G, RPT>(BatchPlace(PLACE), a.nstage, a.width);
     if (PLACE != kGlobalVecs) {
         B2S_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          int(PLACE == kSmemAll ? kMaxBlockSmem - 1024 : sm)));
+                                          int(PLACE == kSmemAll ? kMaxStageSmem : sm)));
     }
     int per_sm = 0;
     B2S_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kBatchBlock, sm));
@@ -450,7 +451,7 @@ int launch_bucket(const BatchConfig& cfg, const BatchArgs& a,
                                                          gscratch_entries, overlap, st); \
         }                                                                      \
         if (batch_smem_bytes<T, GG, RR>(kSmemAll, a.nstage, a.width) <=        \
-            kMaxBlockSmem - 1024) {                                            \
+            kMaxStageSmem) {                                                   \
             return launch_placed<T, GG, RR, kSmemAll>(a, ci, val, b, x, gscratch, \
                                                       gscratch_entries, overlap, st); \
         }                                                                      \

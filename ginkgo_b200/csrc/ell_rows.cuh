@@ -162,6 +162,8 @@ __global__ void __launch_bounds__(256)
 {
     const int64_t s = (blockIdx.x * int64_t(256) + threadIdx.x) / kWarp;
     if (s * kWarp >= n) return;  // whole warp
+    // a slice that was too wide ends the fill early (one answer per warp)
+    if (__any_sync(0xffffffffu, *static_cast<volatile int*>(too_wide))) return;
     const int lane = threadIdx.x % kWarp;
     const int64_t row = s * kWarp + lane;
     T* out = vals + s * width * kWarp + lane;
