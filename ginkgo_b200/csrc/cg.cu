@@ -791,7 +791,8 @@ __global__ void __launch_bounds__(kCgResidentBlock, 1)
     cg_resident_kernel(int64_t n, const int32_t* __restrict__ rp,
                        const int32_t* __restrict__ ci, const T* __restrict__ v,
                        const T* __restrict__ dinv, T* __restrict__ x, int64_t ldx, T* r, T* p0,
-                       T* p1, SolveCtl* ctl, CgScalars<T>* sc, ExchangeSlot* slots, int capacity)
+                       T* p1, SolveCtl* ctl, CgScalars<T>* sc, ExchangeSlot* slots, int capacity,
+                       int polls)
 {
     extern __shared__ __align__(16) unsigned char stage_raw[];
     __shared__ double red[kExchangeShared];
@@ -829,7 +830,7 @@ __global__ void __launch_bounds__(kCgResidentBlock, 1)
     // rows longer than the caller said: all blocks leave together, nothing
     // written
     T over[1] = {threadIdx.x == 0 && cnt > capacity ? T(1) : T(0)};
-    if (!grid_exchange<T, 1>(over, slots, ++epoch, red)) {
+    if (!grid_exchange<T, 1>(over, slots, ++epoch, red, polls)) {
         if (threadIdx.x == 0) ctl->failed = 1;
         return;
     }
@@ -877,7 +878,7 @@ __global__ void __launch_bounds__(kCgResidentBlock, 1)
                 pq[0] += pp[m] * acc;
             }
         }
-        if (!grid_exchange<T, 1>(pq, slots, ++epoch, red)) {
+        if (!grid_exchange<T, 1>(pq, slots, ++epoch, red, polls)) {
             if (threadIdx.x == 0) ctl->failed = 1;
             return;
         }
@@ -894,7 +895,7 @@ __global__ void __launch_bounds__(kCgResidentBlock, 1)
                 sums[1] += rr[m] * rr[m];
             }
         }
-        if (!grid_exchange<T, 2>(sums, slots, ++epoch, red)) {
+        if (!grid_exchange<T, 2>(sums, slots, ++epoch, red, polls)) {
             if (threadIdx.x == 0) ctl->failed = 1;
             return;
         }
@@ -948,8 +949,8 @@ int64_t cg_stage_bytes(int64_t n, int64_t max_row_nnz)
 template <typename T>
 int cg_resident_loop(int64_t n, const int32_t* rp, const int32_t* ci, const T* v, const T* dinv,
                      T* x, int64_t ldx, T* r, T* p0, T* p1, SolveCtl* ctl, CgScalars<T>* sc,
-                     ExchangeSlot* slots, int64_t max_row_nnz, int max_iters, cudaStream_t st,
-                     SolveCtl* host_ctl)
+                     ExchangeSlot* slots, int64_t max_row_nnz, int max_iters, int polls,
+                     cudaStream_t st, SolveCtl* host_ctl)
 {
     // lanes per row while a block's rows still fit its threads: short rows
     // take all their gathers at once
@@ -970,7 +971,7 @@ int cg_resident_loop(int64_t n, const int32_t* rp, const int32_t* ci, const T* v
                                       int(kCgStageBytes)));
     int capacity = int(need / int64_t(sizeof(T) + 4));  // entries of a block's stage
     void* args[] = {&n,  &rp, &ci,  &v,  &dinv,  &x,       &ldx, &r,
-                    &p0, &p1, &ctl, &sc, &slots, &capacity};
+                    &p0, &p1, &ctl, &sc, &slots, &capacity, &polls};
     const int64_t max_launches = int64_t(max_iters) / kCgResidentIters + 2;
     for (int64_t l = 0; l < max_launches; ++l) {
         B2S_CUDA_TRY(cudaMemsetAsync(slots, 0, kExchangeSlots * sizeof(ExchangeSlot), st));
@@ -1169,7 +1170,8 @@ CgLayout cg_layout(int64_t n, int K, bool with_z = false)
     return l;
 }
 
-// bp: a block Jacobi preconditioner (dinv then null), or null
+// bp: a block Jacobi preconditioner (dinv then null), or null.  max_polls:
+// the resident kernel's limit on a wait of its blocks
 template <typename T>
 int cg_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
              int64_t max_row_nnz, const T* dinv, const BlockPrec<T>* bp, const T* b,
@@ -1177,8 +1179,9 @@ int cg_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
              int residual_mode, int64_t check_every, void* workspace,
              int64_t workspace_bytes,
              int64_t* iterations, double* residual_norms, uint8_t* status,
-             void* stream)
+             void* stream, int64_t max_polls = kExchangePolls)
 {
+    B2S_CHECK_ARG(max_polls >= 0 && max_polls < (int64_t(1) << 31), "max_polls out of range");
     B2S_CHECK_ARG(n >= 0 && k >= 1 && k <= kMaxRhs, "num_rhs must be 1..16");
     B2S_CHECK_ARG(ldb >= k && ldx >= k, "leading dimension < num_rhs");
     B2S_CHECK_ARG(max_iters >= 0 && max_iters < (int64_t(1) << 30),
@@ -1349,7 +1352,7 @@ int cg_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
     if (resident) {
         rc = cg_resident_loop<T>(n, rp, ci, v, dinv, x, ldx, r, p[0], p[1], ctl, sc,
                                  reinterpret_cast<ExchangeSlot*>(w + lay.off_slots),
-                                 max_row_nnz, int(max_iters), st, &h);
+                                 max_row_nnz, int(max_iters), int(max_polls), st, &h);
         resident = rc != kCgNotResident;
     }
     if (!resident) rc = run_graph_loop(st, ctl, int(max_iters), chunk, capture, &h);
@@ -1417,6 +1420,22 @@ int64_t b2s_cg_block_workspace_bytes(int64_t num_rows, int64_t num_rhs,
                            check_every, workspace,                            \
                            workspace_bytes, iterations, residual_norms,       \
                            status, stream);                                   \
+    }                                                                         \
+    int b2s_cg_solve_waiting_##S(                                             \
+        int64_t num_rows, const int32_t* row_ptrs, const int32_t* col_idxs,   \
+        const T* values, int64_t max_row_nnz, const T* inv_diag, const T* b,  \
+        int64_t ldb, T* x, int64_t ldx, int64_t num_rhs, int64_t max_iters,   \
+        double reduction_factor, int residual_mode, int64_t check_every,      \
+        void* workspace, int64_t workspace_bytes, int64_t* iterations,        \
+        double* residual_norms, uint8_t* status, void* stream,                \
+        int64_t max_polls)                                                    \
+    {                                                                         \
+        return cg_solve<T>(num_rows, row_ptrs, col_idxs, values, max_row_nnz, \
+                           inv_diag, nullptr, b, ldb, x, ldx, num_rhs,        \
+                           max_iters, reduction_factor, residual_mode,        \
+                           check_every, workspace, workspace_bytes,           \
+                           iterations, residual_norms, status, stream,        \
+                           max_polls);                                        \
     }                                                                         \
     int b2s_cg_block_solve_##S(                                               \
         int64_t num_rows, const int32_t* row_ptrs, const int32_t* col_idxs,  \

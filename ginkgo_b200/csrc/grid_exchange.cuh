@@ -8,8 +8,9 @@ namespace b2s {
 
 // Blocks per exchange: one per SM.
 constexpr int kExchangeBlocks = kMaxSMs;
-// Polls after which a block gives up (each takes a trip to L2, so this is
-// on the order of a second); the kernel then reports the failure and ends.
+// Polls after which a block gives up where the caller does not say (each
+// takes a trip to L2, so this is on the order of a second); the kernel then
+// reports the failure and ends.
 constexpr int kExchangePolls = 1 << 21;
 
 // A block's value and the exchange it belongs to, in two 8-byte words that
@@ -53,8 +54,8 @@ __device__ __forceinline__ void exchange_fence() { asm volatile("fence.acq_rel.g
 // global writes that any thread of the grid made before the call are visible
 // to L2 reads (__ldcg) of every thread.  `epoch` counts the exchanges of the
 // launch from 1; the slots are zero at launch.  False when a block did not
-// arrive in time: the caller ends the kernel.  Threads must be a multiple of
-// 32, up to 1024, at least 64; red holds kExchangeShared values.
+// arrive within `polls` polls: the caller ends the kernel.  Threads must be a
+// multiple of 32, up to 1024, at least 64; red holds kExchangeShared values.
 //
 // Block 0 collects the values and publishes the total, so a waiting block
 // polls one slot.  With every block polling all the others' slots (one hop
@@ -62,7 +63,7 @@ __device__ __forceinline__ void exchange_fence() { asm volatile("fence.acq_rel.g
 // and an exchange took 4.5 to 5 us.
 template <typename T, int M>
 __device__ __forceinline__ bool grid_exchange(T (&v)[M], ExchangeSlot* slots, unsigned epoch,
-                                              double* red)
+                                              double* red, int polls)
 {
     static_assert(M == 1 || M == 2, "one or two values");
     const int lane = threadIdx.x % kWarp, wid = threadIdx.x / kWarp;
@@ -88,7 +89,7 @@ __device__ __forceinline__ bool grid_exchange(T (&v)[M], ExchangeSlot* slots, un
                 exchange_put(buf + blockIdx.x, double(s), epoch);
                 double got = 0.0;
                 all = false;
-                for (int poll = 0; poll < kExchangePolls && !all; ++poll) {
+                for (int poll = 0; poll < polls && !all; ++poll) {
                     all = exchange_get(total, epoch, got);
                 }
                 sum = T(got);
@@ -97,9 +98,9 @@ __device__ __forceinline__ bool grid_exchange(T (&v)[M], ExchangeSlot* slots, un
         } else {
             // block 0 collects: lane l the blocks l, l + 32, ...
             constexpr int kPer = (kExchangeBlocks + kWarp - 1) / kWarp;
-            double got[kPer];
+            double got[kPer] = {};
             all = false;
-            for (int poll = 0; poll < kExchangePolls && !all; ++poll) {
+            for (int poll = 0; poll < polls && !all; ++poll) {
                 bool mine = true;
 #pragma unroll
                 for (int q = 0; q < kPer; ++q) {
@@ -116,8 +117,15 @@ __device__ __forceinline__ bool grid_exchange(T (&v)[M], ExchangeSlot* slots, un
 #pragma unroll
             for (int q = 0; q < kPer; ++q) sum += T(got[q]);
             sum = warp_sum(sum);
-            exchange_fence();  // acquire the others' writes, release with them
-            if (lane == 0 && all) exchange_put(total, double(sum), epoch);
+            // every lane acquires the writes behind the slots it read, and
+            // lane 0 releases them all with the total: shuffles and votes
+            // order no memory between lanes, __syncwarp does
+            exchange_fence();
+            __syncwarp();
+            if (lane == 0 && all) {
+                exchange_fence();
+                exchange_put(total, double(sum), epoch);
+            }
         }
         if (lane == 0) {
             tot[wid] = double(sum);

@@ -605,6 +605,30 @@ int b2s_cg_solve_f32(int64_t num_rows, const int32_t* row_ptrs,
                      void* workspace, int64_t workspace_bytes,
                      int64_t* iterations, double* residual_norms,
                      uint8_t* status, void* stream);
+/* b2s_cg_solve_* with the caller's limit on the waits of a solve that runs as
+ * one cooperative kernel (one right-hand side on a small system): a block that
+ * has polled max_polls times for the others' sums gives up, and the solve ends
+ * with B2S_ERR_CUDA.  b2s_cg_solve_* takes 2^21 polls, about a second. */
+int b2s_cg_solve_waiting_f64(int64_t num_rows, const int32_t* row_ptrs,
+                             const int32_t* col_idxs, const double* values,
+                             int64_t max_row_nnz, const double* inv_diag,
+                             const double* b, int64_t ldb, double* x,
+                             int64_t ldx, int64_t num_rhs, int64_t max_iters,
+                             double reduction_factor, int residual_mode,
+                             int64_t check_every, void* workspace,
+                             int64_t workspace_bytes, int64_t* iterations,
+                             double* residual_norms, uint8_t* status,
+                             void* stream, int64_t max_polls);
+int b2s_cg_solve_waiting_f32(int64_t num_rows, const int32_t* row_ptrs,
+                             const int32_t* col_idxs, const float* values,
+                             int64_t max_row_nnz, const float* inv_diag,
+                             const float* b, int64_t ldb, float* x,
+                             int64_t ldx, int64_t num_rhs, int64_t max_iters,
+                             double reduction_factor, int residual_mode,
+                             int64_t check_every, void* workspace,
+                             int64_t workspace_bytes, int64_t* iterations,
+                             double* residual_norms, uint8_t* status,
+                             void* stream, int64_t max_polls);
 /* CG preconditioned by block Jacobi: num_blocks blocks delimited by
  * block_ptrs (num_blocks + 1 entries covering 0..num_rows, each block at
  * most max_block_size rows), inverses in the interleaved storage that
