@@ -1082,9 +1082,9 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
                         }
                         return;
                     }
-                    launch_rhs_lanes<T, K, 0>(n, rp, 0, 0, nullptr, nullptr, ci, v, in, K, out,
-                                              K, nullptr, nullptr, max_row_nnz, cs,
-                                              &ctl->all_stopped);
+                    rhs_lanes_kernel<T, K, 0><<<ceildiv(n * KL, kLanesBlock), kLanesBlock, 0, cs>>>(
+                        n, rp, 0, 0, nullptr, nullptr, ci, v, in, K, out, K, nullptr, nullptr,
+                        &ctl->all_stopped);
                 } else {
                     with_async_kernel<T, K, (K >= 2)>(lpr, [&](auto kernel) {
                         const int64_t grid = std::min<int64_t>(async_need,

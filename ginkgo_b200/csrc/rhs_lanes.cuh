@@ -232,9 +232,8 @@ __global__ void __launch_bounds__(kLanesBlock)
                     const uint64_t* __restrict__ slice_lengths, const int32_t* __restrict__ ci,
                     const T* __restrict__ v, const T* __restrict__ b, int64_t ldb,
                     T* __restrict__ c, int64_t ldc, const T* __restrict__ alpha,
-                    const T* __restrict__ beta, const int* __restrict__ skip = nullptr)
+                    const T* __restrict__ beta)
 {
-    if (skip != nullptr && *skip) return;
     const int64_t r0 =
         (blockIdx.x * int64_t(kLanesBlock / kWarp) + threadIdx.x / kWarp) * ROWS;
     if (r0 >= n) return;  // whole warp
@@ -245,55 +244,128 @@ __global__ void __launch_bounds__(kLanesBlock)
                               });
 }
 
-// Rows a warp of rhs_rows_kernel takes, 0 where rhs_lanes_kernel stays.
+// Ell with two neighbouring rows per lane slot: the rows' column indices and
+// values at each entry are one 8- or 16-byte vector load (the layout is
+// column-major, so rows r and r + 1 sit next to each other), and each slot
+// gathers two 16-byte pieces of b per entry, eight in flight.  Needs an even
+// stride, vector-aligned indices and values and 16-byte aligned b and c rows;
+// a pair whose second row lies past the matrix computes the first alone.
+template <typename T, int K>
+__global__ void __launch_bounds__(kLanesBlock)
+    rhs_pairs_kernel(int64_t n, int64_t width, int64_t stride, const int32_t* __restrict__ ci,
+                     const T* __restrict__ v, const T* __restrict__ b, int64_t ldb,
+                     T* __restrict__ c, int64_t ldc, const T* __restrict__ alpha,
+                     const T* __restrict__ beta)
+{
+    using V = typename Vec16<T>::type;
+    using V2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+    constexpr int VW = Vec16<T>::width;
+    constexpr int KL = K / VW;
+    const int64_t g = blockIdx.x * int64_t(kLanesBlock) + threadIdx.x;
+    const int64_t r0 = 2 * (g / KL);
+    if (r0 >= n) return;
+    const int sub = int(g % KL);
+    const T* bc = b + sub * VW;
+    V acc0{}, acc1{};
+    const bool second = r0 + 1 < n;  // (r0 + 1 < stride: the stride is even)
+    auto entries = [&](int64_t i, auto count) {
+        constexpr int N = decltype(count)::value;
+        int2 cc[N];
+        V2 vv[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const int64_t e = r0 + (i + u) * stride;
+            cc[u] = __ldg(reinterpret_cast<const int2*>(ci + e));
+            vv[u] = __ldg(reinterpret_cast<const V2*>(v + e));
+        }
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            if (cc[u].x != -1) fma_vec<T>(acc0, vv[u].x, bc + int64_t(cc[u].x) * ldb);
+            if (second && cc[u].y != -1) fma_vec<T>(acc1, vv[u].y, bc + int64_t(cc[u].y) * ldb);
+        }
+    };
+    int64_t i = 0;
+    for (; i + 4 <= width; i += 4) entries(i, std::integral_constant<int, 4>());
+    for (; i < width; ++i) entries(i, std::integral_constant<int, 1>());
+    store_vec<T>(c + r0 * ldc + sub * VW, acc0, alpha, beta);
+    if (second) store_vec<T>(c + (r0 + 1) * ldc + sub * VW, acc1, alpha, beta);
+}
+
+// Rows a warp of rhs_rows_kernel takes; 0 where rhs_lanes_kernel stays, and
+// kRowPairs for rhs_pairs_kernel (Ell, when its alignment allows).
 // `longest`: the longest row (Csr, Ell) or slice (Sellp), 0 when not known.
 //
 // Rows differ in length inside a warp in Csr and Sellp, and a warp runs to
 // its longest: matrices with rows over 64 entries keep rhs_lanes_kernel (one
 // long row holds up the other rows of its warp; the power-law matrix's
-// longest slices have 1,805 entries).  Few rows: the fewest rows per warp,
-// for the most warps (3d 27-point 24^3, 16 FP64 columns, Sellp: 6.9 us with
-// 4 rows, 15.7 with 32).  Many short rows (up to 8 entries, two load steps
-// at most): 32 rows, the longest coalesced loads and stores, except at 16
-// FP64 columns, whose 8 accumulators of 32 rows need 102 registers (267
-// against 231 us with 16 rows, 7-point 128^3).  Longer rows: 16 per warp, so
-// that each load step brings two entries per row (27-point 77^3, 4 FP64
-// columns, Sellp: 55.1 against 65.0 us with 32 rows).
-// 7-point 128^3, 4 / 8 / 16 columns, before -> after: Sellp FP64 141 / 263 /
-// 476 -> 89 / 115 / 231 us, FP32 68 / 133 / 248 -> 47 / 69 / 110 us; Ell FP64
-// 90 / 168 / 318 -> 78 / 128 / 209 us.  Csr's entries of a row already sit
-// together and its reloads hit L1, so there the kernel pays only from four
-// lanes per row on short rows (FP64 117 -> 96 us at 8 columns, 224 -> 204 at
-// 16; FP32 105 -> 85 at 16; at 4 FP64 columns 66 against 69) and on few rows
-// longer than 8 (27-point 24^3, 8 FP64 columns: 7.9 -> 5.5 us).
+// longest slices have 1,805 entries).  Ell's rows are all as long as its
+// width.
+//
+// A warp of many rows makes the longest coalesced loads and stores, which
+// pays once the matrix and the vectors come from HBM: 32 rows when they are
+// short (up to 8 entries, two load steps at most), except at eight lanes per
+// row, whose 8 accumulators of 32 rows need 102 registers (267 against 231 us
+// with 16 rows, 7-point 128^3); 16 longer ones, so that each load step brings
+// two entries per row (27-point 77^3, 4 FP64 columns, Sellp: 55.1 against
+// 65.0 us with 32 rows).  7-point 128^3, 4 / 8 / 16 columns, one row per lane
+// slot (Csr, FP32 4 columns) or two (Ell, Sellp) -> many rows per warp: Sellp
+// FP64 141 / 263 / 474 -> 89 / 115 / 207 us, FP32 67 / 133 / 248 -> 47 / 69 /
+// 110 us; Ell FP64 90 / 167 / 319 -> 78 / 128 / 207 us; Csr (whose entries of
+// a row already sit together and whose reloads hit L1) FP64 115 -> 95 us at 8
+// columns, 224 -> 205 at 16, FP32 104 -> 84 at 16.
+//
+// With fewer rows there are then too few warps to hide the gathers, and the
+// lines below are where the measured sides cross (us, us):
+// - four and eight lanes, Ell and Sellp, few rows: the fewest rows per warp,
+//   which loads several entries of each row per step.  Sellp 27-point 24^3,
+//   16 FP64 columns: 4 rows 6.2, one row per slot 6.4, 16 rows 9.2; 7-point
+//   32^3, 16 FP32 columns: 8 rows 3.5, 32 rows 5.6.
+// - then, for Ell, two rows per lane slot.  27-point 32^3, 16 FP64 columns:
+//   10.2, 16 rows 11.8; 40^3 17.7 and 21.9.  On 2^17 rows the sides meet
+//   (5-point 360^2 9.8, 9.9; 27-point 50^3 37.8, 36.7).
+// - one and two lanes: one row per slot.  27-point 50^3, 4 FP64 columns, Ell:
+//   11.9, 16 rows 14.3.
+// - Csr, short rows: one row per slot up to 2^18 rows at four lanes (7-point
+//   40^3, 16 FP32 columns 4.8, 32 rows 5.3; 64^3 12.2, 11.7) and 2^19 at
+//   eight (7-point 50^3 11.3, 16 rows 12.8; 80^3 55.3, 54.5).
+// - Csr, longer rows: the fewest rows per warp on few rows (27-point 24^3, 8
+//   FP64 columns: 7.9 -> 5.5).
 constexpr int64_t kRowsMaxLen = 64;
-constexpr int64_t kRowsFew = int64_t(1) << 14;
 constexpr int64_t kRowsShort = 8;
+constexpr int kRowPairs = -1;
 
 inline int rhs_rows_per_warp(int fmt, int lanes, int64_t n, int64_t longest)
 {
-    // (Ell's rows are all as long as its width)
-    if (longest <= 0 || longest > (fmt == 1 ? int64_t(1) << 30 : kRowsMaxLen)) return 0;
+    constexpr int64_t k14 = int64_t(1) << 14, k17 = int64_t(1) << 17;
+    if (longest <= 0 || (fmt != 1 && longest > kRowsMaxLen)) return 0;
+    const bool short_rows = longest <= kRowsShort;
     const int fewest = kWarp / lanes;
-    const bool few = n < kRowsFew, short_rows = longest <= kRowsShort;
-    if (fmt == 0 && !(few ? !short_rows : short_rows && lanes >= 4)) return 0;
-    if (few) return fewest;
-    const int rows = short_rows && lanes < 8 ? 32 : 16;
-    return rows > fewest ? rows : fewest;
+    const int many = lanes < 8 && (short_rows || lanes == 1) ? 32 : 16;
+    if (fmt == 0) {
+        if (!short_rows) return n < k14 ? fewest : 0;
+        return lanes == 4 && n >= 2 * k17 ? many : lanes == 8 && n >= 4 * k17 ? many : 0;
+    }
+    if (lanes <= 2) {
+        if (fmt == 1 && lanes == 2 && !short_rows) return 0;
+        return n < (lanes == 2 && short_rows ? k17 / 2 : k17) ? 0 : many;
+    }
+    if (fmt == 1) return n * lanes < k17 ? fewest : n < k17 ? kRowPairs : many;
+    if (lanes == 8 && short_rows) return n < k14 ? fewest : n < 2 * k14 ? 0 : many;
+    return n < k17 / 2 ? fewest : many;
 }
 
-// Calls f(std::integral_constant<int, ROWS>) for a value of
-// rhs_rows_per_warp.
-template <int KL, typename F>
+// Calls f(std::integral_constant<int, ROWS>) for a positive value of
+// rhs_rows_per_warp<FMT>; instances that the rule never picks are not made.
+template <int FMT, int KL, typename F>
 void with_rows_per_warp(int rows, F&& f)
 {
     constexpr int kFewest = kWarp / KL;
     if (rows == kFewest) {
-        f(std::integral_constant<int, kFewest>());
+        if constexpr (FMT != 1 || KL != 2) f(std::integral_constant<int, kFewest>());
     } else if (rows == 32) {
-        if constexpr (KL > 1 && KL < 8) f(std::integral_constant<int, 32>());
+        if constexpr (KL == 4 || (KL == 2 && FMT != 0)) f(std::integral_constant<int, 32>());
     } else {
-        if constexpr (KL > 2) f(std::integral_constant<int, 16>());
+        if constexpr (KL == 8 || (KL == 4 && FMT != 0)) f(std::integral_constant<int, 16>());
     }
 }
 
@@ -303,22 +375,30 @@ template <typename T, int K, int FMT>
 void launch_rhs_lanes(int64_t n, const int32_t* rp, int64_t w_or_s, int64_t stride,
                       const uint64_t* sets, const uint64_t* lens, const int32_t* ci, const T* v,
                       const T* b, int64_t ldb, T* c, int64_t ldc, const T* alpha, const T* beta,
-                      int64_t longest, cudaStream_t st, const int* skip = nullptr)
+                      int64_t longest, cudaStream_t st)
 {
     static_assert(K >= 4 && K % Vec16<T>::width == 0, "column slices of 16 bytes");
     constexpr int KL = K / Vec16<T>::width;
     const int rows = rhs_rows_per_warp(FMT, KL, n, longest);
     if (rows > 0) {
-        with_rows_per_warp<KL>(rows, [&](auto rc) {
+        with_rows_per_warp<FMT, KL>(rows, [&](auto rc) {
             constexpr int ROWS = decltype(rc)::value;
             const int64_t grid = ceildiv(ceildiv(n, ROWS), kLanesBlock / kWarp);
             rhs_rows_kernel<T, K, FMT, ROWS><<<grid, kLanesBlock, 0, st>>>(
-                n, rp, w_or_s, stride, sets, lens, ci, v, b, ldb, c, ldc, alpha, beta, skip);
+                n, rp, w_or_s, stride, sets, lens, ci, v, b, ldb, c, ldc, alpha, beta);
         });
         return;
     }
+    if constexpr (FMT == 1 && KL >= 4) {
+        if (rows == kRowPairs && stride % 2 == 0 && reinterpret_cast<uintptr_t>(ci) % 8 == 0 &&
+            reinterpret_cast<uintptr_t>(v) % (2 * sizeof(T)) == 0) {
+            rhs_pairs_kernel<T, K><<<ceildiv(ceildiv(n, 2) * KL, kLanesBlock), kLanesBlock, 0,
+                                     st>>>(n, w_or_s, stride, ci, v, b, ldb, c, ldc, alpha, beta);
+            return;
+        }
+    }
     rhs_lanes_kernel<T, K, FMT><<<ceildiv(n * KL, kLanesBlock), kLanesBlock, 0, st>>>(
-        n, rp, w_or_s, stride, sets, lens, ci, v, b, ldb, c, ldc, alpha, beta, skip);
+        n, rp, w_or_s, stride, sets, lens, ci, v, b, ldb, c, ldc, alpha, beta);
 }
 
 }  // namespace b2s

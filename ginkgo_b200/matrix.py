@@ -342,8 +342,8 @@ class Sellp(_SparseBase):
         self.slice_sets, self.slice_lengths = slice_sets, slice_lengths
         self.col_idxs, self.values = col_idxs, values
         self.dtype = values.dtype
-        # the longest slice, for the SpMV's choice of one or two rows per
-        # lane slot (read back once here)
+        # the longest slice, for the SpMV's choice of rows per warp (read
+        # back once here)
         self.max_slice_length = int(slice_lengths.max().item()) if slice_lengths.numel() else 0
 
     @property
