@@ -656,6 +656,13 @@ __global__ void __launch_bounds__(kSolverBlock)
     }
 }
 
+// Four FP32 columns are one 16-byte slice: a lane owns a row, and with rows of
+// more than 8 entries the warp's index and value loads of each step lie in 32
+// rows.  From this many rows on they come from HBM and the SpMV with a pass
+// for its dots is shorter (40 iterations, 27-point, dots apart -> fused:
+// 52^3 3.14 -> 2.84 ms, 56^3 3.87 -> 3.73, 64^3 4.24 -> 5.11, 77^3 6.85 -> 8.64).
+constexpr int64_t kBicgApartRows = int64_t(3) << 16;
+
 // q = A in for K columns, a warp per ROWS rows (rhs_rows), with the dots of
 // bicg_dots_lanes_kernel from the finished rows.
 // 20 iterations of the 2D convection-diffusion step, before -> with this pass
@@ -1068,7 +1075,9 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
                 constexpr int NS = decltype(ns)::value;
                 if constexpr (K >= 4 && K % Vec16<T>::width == 0) {
                     constexpr int KL = K / Vec16<T>::width;
-                    if (max_row_nnz >= 1 && max_row_nnz <= kRowsMaxLen) {
+                    const bool apart =
+                        KL == 1 && max_row_nnz > kRowsShort && n >= kBicgApartRows;
+                    if (max_row_nnz >= 1 && max_row_nnz <= kRowsMaxLen && !apart) {
                         // rows per warp as in CG's split iteration
                         auto fused = [&](auto rc) {
                             constexpr int ROWS = decltype(rc)::value;
@@ -1078,7 +1087,7 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
                             kernel<<<pgrid(kernel, gs), kSolverBlock, 0, cs>>>(
                                 n, rp, ci, v, in, out, a, ctl, sc, partials);
                         };
-                        if (KL < 8 && (KL == 1 || max_row_nnz <= kRowsShort)) {
+                        if (KL == 1 || (KL < 8 && max_row_nnz <= kRowsShort)) {
                             fused(std::integral_constant<int, KL < 8 ? 32 : 16>());
                         } else {
                             fused(std::integral_constant<int, KL == 1 ? 32 : 16>());
