@@ -1008,11 +1008,74 @@ int cg_resident_loop(int64_t n, const int32_t* rp, const int32_t* ci, const T* v
 // ||b||^2 (cg::initialize and the first z = M r, core/solver/cg.cpp:
 // 122-149).
 // ---------------------------------------------------------------------------
+// How the last block ends an iteration in the FP64 passes whose registers lie
+// at the edge of two blocks per SM.  kInline is cg_update_finish in place.  In
+// the forms below it pushed the pass past 128 registers, to one block, or into
+// spills: out of line, with two blocks stated, or one thread walking the four
+// columns leaves the pass at 128 (40 iterations, in line -> chosen: 7-point
+// 64^3, blocks of 32 rows, 4 columns 4.08 -> 3.40 ms; 16 rows, 8 columns 4.84
+// -> 4.37 ms; 5-point 1000^2, 16 rows of mixed precisions, 4 columns 6.72 ->
+// 6.45 ms).
+enum CgBlockTail { kInline, kOutOfLine, kOneThread };
+
+template <typename T, int MB2, int K, bool INIT, int SK>
+constexpr CgBlockTail cg_block_tail()
+{
+    if (INIT || sizeof(T) != 8) return kInline;
+    if (K == 8 && (MB2 == 8 || (MB2 == 16 && SK == kSkFull))) return kOutOfLine;
+    if (K == 4 && ((MB2 == 32 && SK == kSkFull) || (MB2 == 16 && SK == kSkMixed))) {
+        return kOneThread;
+    }
+    return kInline;
+}
+
+template <typename T, int K>
+__device__ __noinline__ void cg_block_end(const T* partials, T* tot, T* red, SolveCtl* ctl,
+                                          CgScalars<T>* sc)
+{
+    sum_partials<T, 2 * K>(partials, gridDim.x, tot, red);
+    if (threadIdx.x < kWarp) cg_update_finish<T, K>(tot, ctl, sc);
+}
+
+// cg_update_finish by one thread.
+template <typename T, int K>
+__device__ __forceinline__ void cg_update_finish_serial(const T* tot, SolveCtl* ctl,
+                                                        CgScalars<T>* sc)
+{
+    ctl->ticket = 0;
+    const int iter = ctl->iter + 1;
+    ctl->iter = iter;
+    int all = 1;
+    for (int j = 0; j < K; ++j) {
+        uint8_t s = ctl->status[j];
+        if (!has_stopped(s)) {
+            sc->prev_rho[j] = sc->rho[j];
+            sc->rho[j] = tot[j];
+            sc->tau[j] = sqrt(tot[K + j]);
+            if (residual_met(ctl, sc->tau[j], sc->rho[j], sc->start[j])) {
+                converge_status(s, kResidualId, true);
+            }
+            if (iter >= ctl->max_iters) stop_status(s, kIterationId, true);
+            ctl->status[j] = s;
+        }
+        all &= has_stopped(s);
+    }
+    ctl->all_stopped = all;
+}
+
 // A fixed storage kind widens its loads in registers; holding those
 // instances to five blocks per SM keeps them at the full-precision pass's 48
 // registers (64 otherwise); a minimum of 0 leaves the others unconstrained.
 template <typename T, int MB2, int K, bool INIT, int SK>
-__global__ void __launch_bounds__(kSolverBlock, (MB2 > 8 ? 0 : SK == kF16 ? 6 : SK >= 0 ? 5 : 0))
+constexpr int cg_block_min_blocks()
+{
+    constexpr CgBlockTail tail = cg_block_tail<T, MB2, K, INIT, SK>();
+    if (tail == kOutOfLine || (tail == kOneThread && SK == kSkFull)) return 2;
+    return MB2 > 8 ? 0 : SK == kF16 ? 6 : SK >= 0 ? 5 : 0;
+}
+
+template <typename T, int MB2, int K, bool INIT, int SK>
+__global__ void __launch_bounds__(kSolverBlock, (cg_block_min_blocks<T, MB2, K, INIT, SK>()))
     cg_block_kernel(int64_t n, BlockPrec<T> bp, const T* __restrict__ b, int64_t ldb, int k,
                     T* __restrict__ x, int64_t ldx, T* __restrict__ r, T* __restrict__ z,
                     T* __restrict__ p, const T* __restrict__ q, SolveCtl* ctl,
@@ -1084,12 +1147,17 @@ __global__ void __launch_bounds__(kSolverBlock, (MB2 > 8 ? 0 : SK == kF16 ? 6 : 
     }
     block_partials<T, NS * K>(acc, partials, red);
     if (last_block_done(&ctl->ticket, &last)) {
-        sum_partials<T, NS * K>(partials, gridDim.x, tot, red);
-        if (threadIdx.x < kWarp) {
+        constexpr CgBlockTail tail = cg_block_tail<T, MB2, K, INIT, SK>();
+        if constexpr (tail == kOutOfLine) {
+            cg_block_end<T, K>(partials, tot, red, ctl, sc);
+        } else {
+            sum_partials<T, NS * K>(partials, gridDim.x, tot, red);
             if constexpr (INIT) {
-                cg_init_finish<T, K>(tot, k, ctl, sc);
+                if (threadIdx.x < kWarp) cg_init_finish<T, K>(tot, k, ctl, sc);
+            } else if constexpr (tail == kOneThread) {
+                if (threadIdx.x == 0) cg_update_finish_serial<T, K>(tot, ctl, sc);
             } else {
-                cg_update_finish<T, K>(tot, ctl, sc);
+                if (threadIdx.x < kWarp) cg_update_finish<T, K>(tot, ctl, sc);
             }
         }
     }
