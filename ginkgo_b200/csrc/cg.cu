@@ -1294,7 +1294,10 @@ int cg_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
     const int grid_spmv = int(std::min<int64_t>(row_blocks, solver_grid()));
     const int grid_vec = int(std::min<int64_t>(
         std::max<int64_t>(1, ceildiv(n, kSolverBlock)), solver_grid()));
-    const int chunk = int(std::max<int64_t>(2, (check_every + 1) / 2 * 2));
+    // iterations per replay, even; a solve of fewer records no more than it
+    // runs (7-point 60^3, 4 columns, one iteration: 391 -> 339 us)
+    const int64_t most = std::min<int64_t>(std::max<int64_t>(check_every, 1), max_iters);
+    const int chunk = int(std::max<int64_t>(2, (most + 1) / 2 * 2));
 
     B2S_DISPATCH_RHS(K, {
         B2S_DISPATCH_SW(sw, {
