@@ -500,6 +500,7 @@ int launch_bucket(const BatchConfig& cfg, const BatchArgs& a,
     B2S_BATCH_CASE(256, 1)
     B2S_BATCH_CASE(256, 2)
     B2S_BATCH_CASE(256, 4)
+    B2S_BATCH_CASE(256, 8)
 #undef B2S_BATCH_CASE
     set_error("unsupported batch configuration G=%d RPT=%d", cfg.G, cfg.RPT);
     return B2S_ERR_UNSUPPORTED;
