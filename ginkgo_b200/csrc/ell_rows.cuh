@@ -193,15 +193,17 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// (FP32 at six blocks per SM: 31.7 -> 30.1 us on 27-point 96^3)
-constexpr int kSliceBatch = 9;
-
 // y = A x over that layout, a thread per row: a slice's offsets are one
 // coalesced load (of the warp's next slice while this one is summed), handed
 // on by shuffles; its values and its x entries at every slot are one
 // contiguous stretch each.  Entries are summed in stored order.
-template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4)
+//
+// B slots are in flight at a time.  Slots past the width repeat the last one
+// with a zero value, so B is the width where it is 5 or 7 (rows of the 5- and
+// 7-point stencils) and 9, a third of a 27-point row, otherwise.  (Nine FP32
+// slots fit five blocks per SM; six spill 24 bytes and are no faster.)
+template <typename T, int B>
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : B == 9 ? 5 : 6)
     slice_rows_kernel(int64_t n, int width, const int32_t* __restrict__ offs,
                       const T* __restrict__ vals, const T* __restrict__ x, T* __restrict__ y,
                       const int* __restrict__ skip)
@@ -222,28 +224,44 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 4)
         for (int k0 = 0; k0 < width; k0 += kWarp) {
             const int cnt = width - k0 < kWarp ? width - k0 : kWarp;
             if (k0 > 0 && lane < cnt) off = __ldg(offs + s * width + k0 + lane);
-            // kSliceBatch slots at a time, all their loads unconditional (a
-            // conditional load here is a branch, and the slots then run one
-            // by one): past the width the last slot with a zero value, and
-            // for a slot that points outside x, which no row of it fills,
-            // the last entry
-            for (int k = 0; k < cnt; k += kSliceBatch) {
-                T v[kSliceBatch], xv[kSliceBatch];
+            // all loads unconditional (a conditional load here is a branch,
+            // and the slots then run one by one): past the width the last
+            // slot with a zero value, and for a slot that points outside x,
+            // which no row of it fills, the last entry
+            for (int k = 0; k < cnt; k += B) {
+                T v[B], xv[B];
 #pragma unroll
-                for (int u = 0; u < kSliceBatch; ++u) {
+                for (int u = 0; u < B; ++u) {
                     const int kk = k + u < cnt ? k + u : cnt - 1;
                     const unsigned c = row + unsigned(__shfl_sync(0xffffffffu, off, kk));
                     v[u] = __ldcs(vp + kk * kWarp);
                     xv[u] = __ldg(x + (c < rows ? c : rows - 1));
                 }
 #pragma unroll
-                for (int u = 0; u < kSliceBatch; ++u) {
+                for (int u = 0; u < B; ++u) {
                     acc += (k + u < cnt ? v[u] : T(0)) * xv[u];
                 }
             }
             vp += int64_t(cnt) * kWarp;
         }
         if (row < rows) y[row] = acc;
+    }
+}
+
+// Calls f(slice_rows_kernel<T, B>) for rows of `width` slots.  Product on the
+// Ell copy -> here, nine slots at a time -> by width: 5-point 700^2 FP64 9.1 ->
+// 9.6 -> 8.5 us, FP32 9.3 -> 9.2 -> 7.1; 7-point 96^3 FP64 18.3 -> 14.9 -> 13.8,
+// 80^3 FP32 11.1 -> 9.6 -> 7.8; 27-point 96^3 FP64 48.3 -> 37.1, 64^3 FP32 24.0
+// -> 13.4.
+template <typename T, typename F>
+void with_slice_batch(int width, F&& f)
+{
+    if (width <= 5) {
+        f(slice_rows_kernel<T, 5>);
+    } else if (width <= 7) {
+        f(slice_rows_kernel<T, 7>);
+    } else {
+        f(slice_rows_kernel<T, 9>);
     }
 }
 

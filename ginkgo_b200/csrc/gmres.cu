@@ -1233,9 +1233,10 @@ int gmres_engine(const GmresLayout& lay, int64_t n, int64_t nnz, const int32_t* 
             // or by the previous step's update
             TA* dst = wbuf;
             if (sliced) {
-                auto kernel = slice_rows_kernel<TA>;
-                kernel<<<pgrid(kernel, std::max<int64_t>(1, ceildiv(n, 256))), 256, 0, cs>>>(
-                    n, ell_w, ell_c, ell_v, y, dst, &gs->idle);
+                with_slice_batch<TA>(ell_w, [&](auto kernel) {
+                    kernel<<<pgrid(kernel, std::max<int64_t>(1, ceildiv(n, 256))), 256, 0, cs>>>(
+                        n, ell_w, ell_c, ell_v, y, dst, &gs->idle);
+                });
             } else if (ell_w > 0) {
                 const int16_t* c16 = reinterpret_cast<const int16_t*>(ell_c);
                 if (ell_r == kEllRows && ell16) {
