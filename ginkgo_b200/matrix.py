@@ -41,12 +41,16 @@ class CudaExecutor:
         torch.cuda.synchronize(self.device)
 
 
+# torch's own accessor of the current stream's handle, where this torch has it
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(t: torch.Tensor):
     # the handle alone: a torch.cuda.Stream object costs about 1.5 us
-    index = t.device.index
-    if index is None:  # not a CUDA tensor: raises
+    if _raw_stream is None or t.device.index is None:
+        # (raises for a tensor that is not on a GPU)
         return torch.cuda.current_stream(t.device).cuda_stream
-    return torch._C._cuda_getCurrentRawStream(index)
+    return _raw_stream(t.device.index)
 
 
 def _p(t):
