@@ -20,18 +20,22 @@
 //
 // p and v are double-buffered so every row reads the previous iterate.
 //
-// One right-hand side on a large system runs the two SpMV passes split, so
-// the matrix streams through the pipelined Csr kernel with one gather per
-// stored entry (forming p' and s at every gathered column triples the
-// gathers once the vectors no longer sit in L2); four or more right-hand
-// sides always run split, with the column-slice SpMV (bicg_vec_k_kernel,
-// rhs_lanes_kernel, bicg_dot1k/2k_kernel), as does block Jacobi:
-//   bicg_pupdate  p' and y = D^-1 p'      csr_async  v = A y
-//   bicg_dot1     dot(rr, v) -> alpha      bicg_supdate  s, z = D^-1 s
-//   csr_async     t = A z                  bicg_dot2  dot(s, t), dot(t, t),
-//                                          ||s|| -> the check on s, omega
-// then the update pass as above.  Every vector entry is rounded as in the
-// fused passes.
+// One right-hand side on a large system (2^19 rows), four or more right-hand
+// sides, and block Jacobi form p' and s in passes of their own, so that an
+// SpMV gathers one vector per stored entry and the matrix streams (forming
+// them at every gathered column triples the gathers once the vectors no
+// longer sit in L2):
+//   p' and y = D^-1 p'    bicg_pupdate_kernel (one column), bicg_vec_lanes_kernel
+//                         (column slices), bicg_block_vec_kernel (block Jacobi)
+//   v = A y, dot(rr, v)   -> alpha
+//   s and z = D^-1 s      as p'
+//   t = A z, dot(s, t), dot(t, t), ||s||^2 -> the check on s, omega
+// then the update pass as above.  The dots come out of the SpMV: as the
+// epilogue of the pipelined Csr kernel (one column, BicgDotEpilogue) or from
+// the finished rows of bicg_spmv_rows_kernel (column slices, rows of up to 64
+// entries); longer rows, four FP32 columns with long rows on large systems, and
+// two or three columns with block Jacobi take them in a pass of their own.
+// Every vector entry is rounded as in the fused passes.
 #include "csr_async.cuh"
 #include "jacobi_scheme.cuh"
 #include "rhs_lanes.cuh"
@@ -468,47 +472,6 @@ __global__ void __launch_bounds__(kSolverBlock)
         const T sr = bicg_s(r[i], v[i], alpha);
         s[i] = sr;
         z[i] = dinv ? mul_rn(dinv[i], sr) : sr;
-    }
-}
-
-// The split passes' vector updates for K columns (several right-hand
-// sides): STEP 1 p' = r + tmp (p - omega v) and y = D^-1 p'; STEP 2
-// s = r - alpha v and z = D^-1 s.  Stopped columns are left as they are.
-template <typename T, int K, int STEP>
-__global__ void __launch_bounds__(kSolverBlock)
-    bicg_vec_k_kernel(int64_t n, const T* __restrict__ dinv, const T* __restrict__ r,
-                      const T* __restrict__ a_old, const T* __restrict__ v_old,
-                      T* __restrict__ out, T* __restrict__ prec, SolveCtl* ctl,
-                      BicgScalars<T>* sc)
-{
-    if (ctl->all_stopped) return;
-    bool active[K], from_r[K];
-    T c1[K], c2[K];
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-        active[j] = !has_stopped(ctl->status[j]);
-        if (STEP == 1) {
-            c2[j] = sc->omega[j];
-            from_r[j] = sc->prev_rho[j] * c2[j] == T(0);
-            c1[j] = from_r[j] ? T(0) : sc->rho[j] / sc->prev_rho[j] * sc->alpha[j] / c2[j];
-        } else {
-            from_r[j] = false;
-            c1[j] = sc->alpha[j];
-            c2[j] = T(0);
-        }
-    }
-    for (int64_t i = blockIdx.x * int64_t(kSolverBlock) + threadIdx.x; i < n;
-         i += int64_t(gridDim.x) * kSolverBlock) {
-        const T d = dinv ? dinv[i] : T(1);
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            if (!active[j]) continue;
-            const int64_t e = i * K + j;
-            const T val = STEP == 1 ? bicg_p(r[e], a_old[e], v_old[e], c1[j], c2[j], from_r[j])
-                                    : bicg_s(r[e], a_old[e], c1[j]);
-            out[e] = val;
-            prec[e] = dinv ? mul_rn(d, val) : val;
-        }
     }
 }
 
@@ -1130,18 +1093,12 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
             } else if constexpr (kLanes) {
                 bicg_vec_lanes_kernel<T, K, 1><<<pgrid(bicg_vec_lanes_kernel<T, K, 1>, grid_lanes), kSolverBlock, 0, cs>>>(
                     n, dinv, r, p[o], vv[o], p[nw], yv, ctl, sc);
-            } else {
-                bicg_vec_k_kernel<T, K, 1><<<pgrid(bicg_vec_k_kernel<T, K, 1>, grid_vec), kSolverBlock, 0, cs>>>(
-                    n, dinv, r, p[o], vv[o], p[nw], yv, ctl, sc);
             }
             spmv_k(yv, vv[nw], rr, alpha_dot);
             if (bp) {
                 launch_bicg_block_vec<T, K, 2>(n, *bp, r, vv[nw], nullptr, s, zv, ctl, sc, cs);
             } else if constexpr (kLanes) {
                 bicg_vec_lanes_kernel<T, K, 2><<<pgrid(bicg_vec_lanes_kernel<T, K, 2>, grid_lanes), kSolverBlock, 0, cs>>>(
-                    n, dinv, r, vv[nw], nullptr, s, zv, ctl, sc);
-            } else {
-                bicg_vec_k_kernel<T, K, 2><<<pgrid(bicg_vec_k_kernel<T, K, 2>, grid_vec), kSolverBlock, 0, cs>>>(
                     n, dinv, r, vv[nw], nullptr, s, zv, ctl, sc);
             }
             spmv_k(zv, t, s, omega_dots);
@@ -1176,15 +1133,17 @@ int bicgstab_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
                 continue;
             }
             B2S_DISPATCH_RHS(K, {
-                B2S_DISPATCH_SW(sw, {
-                    bicg_spmv1_kernel<T, SW, K><<<pgrid(bicg_spmv1_kernel<T, SW, K>, grid_spmv), kSolverBlock, 0, cs>>>(
-                        n, rp, ci, v, dinv, r, rr, p[o], vv[o], p[nw], vv[nw],
-                        ctl, sc, partials);
-                    bicg_spmv2_kernel<T, SW, K><<<pgrid(bicg_spmv2_kernel<T, SW, K>, grid_spmv), kSolverBlock, 0, cs>>>(
-                        n, rp, ci, v, dinv, r, vv[nw], s, t, ctl, sc, partials);
-                });
-                bicg_update_kernel<T, K><<<pgrid(bicg_update_kernel<T, K>, grid_vec), kSolverBlock, 0, cs>>>(
-                    n, dinv, x, ldx, r, rr, p[nw], s, t, ctl, sc, partials);
+                if constexpr (K < 4) {  // (four and more run split)
+                    B2S_DISPATCH_SW(sw, {
+                        bicg_spmv1_kernel<T, SW, K><<<pgrid(bicg_spmv1_kernel<T, SW, K>, grid_spmv), kSolverBlock, 0, cs>>>(
+                            n, rp, ci, v, dinv, r, rr, p[o], vv[o], p[nw], vv[nw],
+                            ctl, sc, partials);
+                        bicg_spmv2_kernel<T, SW, K><<<pgrid(bicg_spmv2_kernel<T, SW, K>, grid_spmv), kSolverBlock, 0, cs>>>(
+                            n, rp, ci, v, dinv, r, vv[nw], s, t, ctl, sc, partials);
+                    });
+                    bicg_update_kernel<T, K><<<pgrid(bicg_update_kernel<T, K>, grid_vec), kSolverBlock, 0, cs>>>(
+                        n, dinv, x, ldx, r, rr, p[nw], s, t, ctl, sc, partials);
+                }
             });
             B2S_LAUNCH_CHECK();
         }
