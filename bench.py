@@ -906,9 +906,9 @@ def batch_section(exe, stream, num_systems=8192, seed=3):
         bn.index_add_(0, seg, b.double() ** 2)
         rel = s.logger.residual_norms / bn.sqrt()
         vb = 8 if dt == torch.float64 else 4
-        # two matrix reads per iteration (5 slots per row, value + index)
-        mat_bytes = float((it * torch.from_numpy(np.diff(A.host_row_offsets)).cuda()
-                           .double()).sum()) * 2 * 5 * (vb + 4)
+        # the matrices once per solve (5 slots per row, value + index): they
+        # stay in shared memory for the iterations
+        mat_bytes = float(A.total_rows) * 5 * (vb + 4)
         buckets = {f"<={1 << k}": {"threads_per_system": int(table[2 * k]),
                                    "vectors_in_smem": bool(table[2 * k + 1])}
                    for k in range(12) if table[2 * k] > 0}

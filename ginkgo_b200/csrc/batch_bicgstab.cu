@@ -122,10 +122,11 @@ constexpr int batch_vec_entries()
 }
 
 // Resident blocks the registers are held to: three 256-thread blocks are
-// also what the stages of the largest bucket leave room for (67 KB each at
+// also what the stages of the largest bucket leave room for (60 KB each at
 // 1024 rows of five FP64 entries), and the group's barriers and reductions
-// need other groups to hide behind (one block per SM at 130 registers: 6.3
-// ms on the workload above).
+// need other groups to hide behind (one block per SM at 130 registers: 6.3 ms
+// on the 8192 systems below).  At 80 registers the FP64 forms of four rows per
+// thread spill 52 to 108 bytes.
 // The forms that read the matrix from global memory are left unconstrained.
 template <typename T, int RPT, int PLACE>
 constexpr int batch_min_blocks()

@@ -749,11 +749,13 @@ __global__ void __launch_bounds__(kSolverBlock)
 // preconditioned vectors M p' and M s are no longer row-wise scales, so the
 // iteration runs split for any number of right-hand sides:
 //   bicg_block_vec  p' = r + tmp (p - omega v) and y = M p'   (STEP 1)
-//   csr_async       v = A y
-//   bicg_dot1k      dot(rr, v) -> alpha
+//   SpMV            v = A y
+//   dot(rr, v)      -> alpha
 //   bicg_block_vec  s = r - alpha v and z = M s             (STEP 2)
-//   csr_async       t = A z
-//   bicg_dot2k      dot(s, t), dot(t, t), ||s|| -> check on s, omega
+//   SpMV            t = A z
+//   dot(s, t), dot(t, t), ||s|| -> check on s, omega
+// (the SpMVs and dots as listed at the top: column slices from four columns
+// on, else csr_async with bicg_dot1k and bicg_dot2k)
 //   bicg_update     x += alpha y + omega z, r = s - omega t (zs = z)
 // bicg_block_vec runs one warp per group of the block-interleaved storage,
 // lane (sub, i) owning row i of block sub: the block's lanes form their

@@ -629,7 +629,7 @@ struct CgDotEpilogue {
     }
 };
 
-// q = A p for K columns, a warp per 32 rows (rhs_rows), with dot(p, q) per
+// q = A p for K columns, a warp per 16 or 32 rows (rhs_rows), with dot(p, q) per
 // column from the finished rows.
 template <typename T, int K, int ROWS>
 __global__ void __launch_bounds__(kSolverBlock)
@@ -777,7 +777,7 @@ __global__ void __launch_bounds__(kSolverBlock)
 // threads) owns RPT rows and keeps their r, x, p, q and D^-1 in registers;
 // r and p go to global memory only for the other rows' gathers, which read
 // L2 (__ldcg), p double buffered as in the fused passes.
-// 5-point 256^2 to 1e-10 (710 iterations): 11.7 -> 5.8 ms.
+// 5-point 256^2 to 1e-10 (710 iterations): 11.3 -> 6.0 ms.
 // ---------------------------------------------------------------------------
 constexpr int kCgResidentBlock = 512;
 constexpr int kCgResidentIters = 1 << 13;  // iterations per launch
@@ -1196,8 +1196,8 @@ void launch_cg_block(int64_t n, const BlockPrec<T>& bp, const T* b, int64_t ldb,
 // Whether one column runs the resident kernel: four rows per thread at most
 // (303,104 rows on 148 SMs) and the entries of a block's rows in its shared
 // memory.  100 iterations, passes -> resident, us per iteration: 5-point 64^2
-// 17.1 -> 7.7, 256^2 19.6 -> 8.9, 512^2 26.0 -> 14.0; 7-point 20^3 16.7 ->
-// 9.0, 67^3 (the largest) 29.0 -> 15.8; 27-point 40^3 27.7 -> 12.3.  With the
+// 16.5 -> 8.0, 256^2 18.5 -> 8.8, 512^2 25.6 -> 13.1; 7-point 20^3 16.3 ->
+// 10.4, 67^3 (the largest) 28.7 -> 16.6; 27-point 40^3 27.2 -> 12.5.  With the
 // entries left in L2 the 27-point 64^3 system took 53.6 us against 38.4 in
 // the split passes.
 template <typename T>
@@ -1316,7 +1316,7 @@ int cg_solve(int64_t n, const int32_t* rp, const int32_t* ci, const T* v,
     });
     // the split iteration: one column of a large system, or four and more
     // (16-byte column slices) whose rows are short enough for a warp to
-    // walk 32 of them together
+    // walk 16 or 32 of them together
     const int lpr = async_lanes_per_row(max_row_nnz);
     const int64_t async_need = ceildiv(ceildiv(n, kWarp / lpr), kAsyncBlock / kWarp);
     const bool split1 = K == 1 && n >= kCgSplitRows;

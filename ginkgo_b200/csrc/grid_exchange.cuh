@@ -119,7 +119,8 @@ __device__ __forceinline__ bool grid_exchange(T (&v)[M], ExchangeSlot* slots, un
             sum = warp_sum(sum);
             // every lane acquires the writes behind the slots it read, and
             // lane 0 releases them all with the total: shuffles and votes
-            // order no memory between lanes, __syncwarp does
+            // order no memory between lanes, __syncwarp does (0.15 us of
+            // each exchange: CG on 5-point 256^2, 710 iterations, 5.8 -> 6.0 ms)
             exchange_fence();
             __syncwarp();
             if (lane == 0 && all) {

@@ -555,13 +555,21 @@ int b2s_residual_norm_check_f32(int64_t k, const float* tau,
 /* Whole-solve entry points.  They run the reference's solver loop on the
  * device with fused kernels and no host synchronisation inside an
  * iteration; the host checks the device stop flag once per replay of a
- * captured CUDA graph.  They synchronise `stream` before returning and
- * write the host outputs (iterations, residual norms, status).  Stopping:
- * Iteration(max_iters) + a residual criterion per right-hand-side column,
- * ||r|| <= reduction_factor * baseline, chosen by residual_mode (below);
- * status[j] uses the bit layout of
- * gko::stopping_status (include/ginkgo/core/stop/stopping_status.hpp):
- * bit 7 converged, bit 6 finalized, bits 0-5 criterion id (1 iteration
+ * captured CUDA graph of at most check_every iterations (rounded up to an
+ * even number).  CG with one right-hand side and no block preconditioner, up
+ * to four rows per thread of one 512-thread block per SM (303,104 rows on 148
+ * SMs) whose entries fit the blocks' shared memory, runs as one cooperative
+ * kernel instead, 8,192 iterations per look, whatever check_every says: its
+ * blocks take a whole SM each (one SM per 32 rows, up to all), so it starts
+ * once other streams' kernels have left those SMs, and such solves on several
+ * streams follow one another.  A kernel on another stream must therefore not
+ * wait for such a solve while it holds an SM. They synchronise `stream`
+ * before returning and write the host outputs (iterations, residual norms,
+ * status). Stopping: Iteration(max_iters) + a residual criterion per right-
+ * hand-side column, ||r|| <= reduction_factor * baseline, chosen by
+ * residual_mode (below); status[j] uses the bit layout of
+ * gko::stopping_status (include/ginkgo/core/stop/stopping_status.hpp): bit 7
+ * converged, bit 6 finalized, bits 0-5 criterion id (1 iteration
  * limit, 2 residual norm).  inv_diag: scalar Jacobi (from
  * b2s_jacobi_invert_diagonal_*) or NULL for no preconditioner. */
 
@@ -854,7 +862,9 @@ int b2s_csr_sddmm_f32(int64_t num_rows, const int32_t* row_ptrs,
  * offsets in host memory (used to sort systems into size buckets).
  * tune_table: NULL for the built-in choice, or 24 int32 from
  * b2s_batch_ell_bicgstab_tune_* (per size bucket 2^k rows: threads per
- * system, 1 = vectors in shared memory / 0 = global scratch).  Synchronises
+ * system; 1 = the product's input vector in shared memory, with the systems'
+ * matrices staged beside it where two such blocks fit an SM, 0 = the vector in
+ * the global scratch and the matrices in global memory).  Synchronises
  * the stream.  Replaces batch_bicgstab::apply
  * (core/solver/batch_bicgstab_kernels.hpp:177-190;
  * cuda/solver/batch_bicgstab_kernels.cu:24-153). */
